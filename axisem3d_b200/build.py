@@ -2,8 +2,8 @@
 
     python -m axisem3d_b200.build          # or __graft_entry__.build()
 
-nvcc cross-compiles for sm_100a without a GPU. The three precision engines are
-separate translation units compiled in parallel; the result is linked with the
+nvcc cross-compiles for sm_100a without a GPU. The three precision engines and the solid
+kernels of each (precision, rheology) pair are separate translation units compiled in parallel; the result is linked with the
 static CUDA runtime so the library only needs the driver at run time.
 """
 import os
@@ -22,6 +22,9 @@ CU_FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xc
                    "-diag-suppress", "607"]
 CU_SOURCES = ["engine_fp32.cu", "engine_fp64.cu", "engine_mixed.cu", "noalloc.cu"]
 CPP_SOURCES = ["capi.cpp", "operands.cpp"]
+# solid_inst.cu is compiled once per (precision, rheology): the longest compilations first
+SOLID_INST = [("solid_%s_%s" % (p, r), t, at, i) for r, i in (("tiso", 1), ("aniso", 2), ("iso", 0))
+              for p, t, at in (("fp64", "double", "double"), ("mixed", "float", "double"), ("fp32", "float", "float"))]
 
 
 def _sources():
@@ -48,6 +51,10 @@ def build(force=False, verbose=False):
         return OUT
     os.makedirs(BUILD, exist_ok=True)
     jobs = []
+    for name, t, at, rheo in SOLID_INST:
+        jobs.append([NVCC] + CU_FLAGS + ["-DAXG_INST_T=" + t, "-DAXG_INST_AT=" + at, "-DAXG_INST_RHEO=%d" % rheo,
+                                         "-c", os.path.join(CSRC, "solid_inst.cu"), "-o",
+                                         os.path.join(BUILD, name + ".o")])
     for src in CU_SOURCES:
         obj = os.path.join(BUILD, src.replace(".cu", ".o"))
         jobs.append([NVCC] + CU_FLAGS + ["-c", os.path.join(CSRC, src), "-o", obj])
@@ -59,7 +66,8 @@ def build(force=False, verbose=False):
         for r in ex.map(_run, jobs):
             if verbose and r.stderr:
                 sys.stderr.write(r.stderr)
-    objs = [os.path.join(BUILD, s.replace(".cu", ".o")) for s in CU_SOURCES] + \
+    objs = [os.path.join(BUILD, n[0] + ".o") for n in SOLID_INST]
+    objs += [os.path.join(BUILD, s.replace(".cu", ".o")) for s in CU_SOURCES] + \
            [os.path.join(BUILD, s.replace(".cpp", ".o")) for s in CPP_SOURCES]
     tmp = OUT + ".tmp"
     _run([NVCC] + ARCH + ["-shared", "-o", tmp] + objs + ["-cudart", "static"])

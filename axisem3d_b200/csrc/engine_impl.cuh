@@ -12,8 +12,7 @@
 #include "adjoint_kernel.cuh"
 #include "fluid_kernel.cuh"
 #include "point_kernels.cuh"
-#include "prt_kernel.cuh"
-#include "solid_kernel.cuh"
+#include "solid_pick.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -1109,73 +1108,6 @@ private:
     }
 
     // ------------------------------------------------------- solid buckets ---
-    using SolidKernel = void (*)(const SolidArgs<T, AT>, int, int, int, int, size_t);
-    // NS: the register-resident SLS recursions are built for 3 and 5 SLS (3-D slices and
-    // 1-D Fourier slots); other counts take the generic path
-    template <int RHEO, int ATT, bool IS3D, bool RTZ>
-    static SolidKernel pick4(int nsls, bool fft) {
-#ifndef AXG_GENERIC_SLS_ONLY
-        if constexpr (ATT != ATT_NONE) {
-            if constexpr (IS3D) {
-                if (fft && nsls == 3) return solid_stiffness_kernel<T, AT, RHEO, ATT, IS3D, RTZ, 3, true>;
-                if (fft && nsls == 5) return solid_stiffness_kernel<T, AT, RHEO, ATT, IS3D, RTZ, 5, true>;
-            }
-            if (nsls == 3) return solid_stiffness_kernel<T, AT, RHEO, ATT, IS3D, RTZ, 3>;
-            if (nsls == 5) return solid_stiffness_kernel<T, AT, RHEO, ATT, IS3D, RTZ, 5>;
-        }
-#endif
-        if constexpr (IS3D && ATT == ATT_NONE) {
-            if (fft) return solid_stiffness_kernel<T, AT, RHEO, ATT, IS3D, RTZ, 0, true>;
-        }
-        return solid_stiffness_kernel<T, AT, RHEO, ATT, IS3D, RTZ, 0>;
-    }
-    template <int RHEO, int ATT, bool IS3D>
-    static SolidKernel pick3(bool rtz, int nsls, bool fft) {
-        if constexpr (RHEO == RHEO_ISO) return pick4<RHEO, ATT, IS3D, false>(nsls, fft);
-        else return rtz ? pick4<RHEO, ATT, IS3D, true>(nsls, fft) : pick4<RHEO, ATT, IS3D, false>(nsls, fft);
-    }
-    template <int RHEO, int ATT>
-    static SolidKernel pick2(bool is3d, bool rtz, int nsls, bool fft) {
-        return is3d ? pick3<RHEO, ATT, true>(rtz, nsls, fft) : pick3<RHEO, ATT, false>(rtz, nsls, fft);
-    }
-    template <int RHEO>
-    static SolidKernel pick1(int att, bool is3d, bool rtz, int nsls, bool fft) {
-        switch (att) {
-            case ATT_NONE: return pick2<RHEO, ATT_NONE>(is3d, rtz, nsls, fft);
-            case ATT_FULL: return pick2<RHEO, ATT_FULL>(is3d, rtz, nsls, fft);
-            default: return pick2<RHEO, ATT_CG4>(is3d, rtz, nsls, fft);
-        }
-    }
-    static SolidKernel pick_solid(int rheo, int att, bool is3d, bool rtz, int nsls, bool fft) {
-        switch (rheo) {
-            case RHEO_ISO: return pick1<RHEO_ISO>(att, is3d, rtz, nsls, fft);
-            case RHEO_TISO: return pick1<RHEO_TISO>(att, is3d, rtz, nsls, fft);
-            default: return pick1<RHEO_ANISO>(att, is3d, rtz, nsls, fft);
-        }
-    }
-
-    using PrtKernel = void (*)(const PrtArgs<T, AT>, int, int, int, size_t);
-    template <int RHEO, int ATT>
-    static PrtKernel pick_prt2(bool is3d, bool rtz) {
-        if (is3d) return rtz ? solid_prt_kernel<T, AT, RHEO, ATT, true, true> : solid_prt_kernel<T, AT, RHEO, ATT, true, false>;
-        return rtz ? solid_prt_kernel<T, AT, RHEO, ATT, false, true> : solid_prt_kernel<T, AT, RHEO, ATT, false, false>;
-    }
-    template <int RHEO>
-    static PrtKernel pick_prt1(int att, bool is3d, bool rtz) {
-        switch (att) {
-            case ATT_NONE: return pick_prt2<RHEO, ATT_NONE>(is3d, rtz);
-            case ATT_FULL: return pick_prt2<RHEO, ATT_FULL>(is3d, rtz);
-            default: return pick_prt2<RHEO, ATT_CG4>(is3d, rtz);
-        }
-    }
-    static PrtKernel pick_prt(int rheo, int att, bool is3d, bool rtz) {
-        switch (rheo) {
-            case RHEO_ISO: return pick_prt1<RHEO_ISO>(att, is3d, rtz);
-            case RHEO_TISO: return pick_prt1<RHEO_TISO>(att, is3d, rtz);
-            default: return pick_prt1<RHEO_ANISO>(att, is3d, rtz);
-        }
-    }
-
     int nmod_of(int rheo) const { return rheo == RHEO_ISO ? 2 : rheo == RHEO_TISO ? 5 : 21; }
 
     // Colour of every element for deterministic assembly (axg_config.deterministic): greedy, in
@@ -1334,13 +1266,13 @@ private:
             state_offs.push_back(soff);
             if (b->prt) {
                 b->xpool.upload(xpool); b->xoff.upload(xoff); b->x3d.upload(x3d);
-                b->pkernel = pick_prt(b->rheo, b->att, b->is3d, b->rtz);
+                b->pkernel = pick_prt<T, AT>(b->rheo, b->att, b->is3d, b->rtz);
             } else {
                 // the slice FFTs: batched 3-D buckets of the register-resident slice path that
                 // hold an nr of at least AXG_FFT_MIN_NR (the plain method keeps the direct sums)
                 const bool reg_path = b->att == ATT_NONE || cfg_.nsls == 3 || cfg_.nsls == 5;
                 b->fft = (!cfg_.plain && b->is3d && reg_path && AXG_FFT_MIN_NR > 0 && b->nr_max >= AXG_FFT_MIN_NR) ? 1 : 0;
-                b->kernel = pick_solid(b->rheo, b->att, b->is3d, b->rtz, cfg_.nsls, b->fft != 0);
+                b->kernel = pick_solid<T, AT>(b->rheo, b->att, b->is3d, b->rtz, cfg_.nsls, b->fft != 0);
             }
             configure_bucket(*b);
             sb_.push_back(std::move(b));

@@ -102,6 +102,9 @@ class Engine final : public EngineBase {
         int n = 0, ndim = 3, total = 0, n3d = 0, nr_max = 1;
         std::vector<int> h_off, h_nu, h_nr;
         std::vector<uint8_t> h_flags;
+        std::vector<T> h_inv1;
+        DBuf<uint8_t> mode_flags;
+        DBuf<T> mode_inv;
         DBuf<int> off, nu, nr, mode_pt, pt3d;
         DBuf<uint8_t> flags;
         DBuf<T> inv1, inv3;
@@ -179,6 +182,8 @@ public:
         build_points(m.sp, sp_, true);
         build_points(m.fp, fp_, false);
         build_ocean(m);
+        upload_mode_tables(sp_, true);
+        upload_mode_tables(fp_, false);
         // twiddles for every nr in use (3-D elements and Mass3D points)
         std::vector<int> nrs;
         int nrmax = 1;
@@ -1091,6 +1096,7 @@ private:
         P.mode_pt.upload(mode_pt); P.pt3d.upload(pt3d);
         P.flags.upload(flags); P.inv1.upload(inv1);
         P.h_flags = flags;
+        P.h_inv1 = inv1;
         if (inv3.empty()) inv3.push_back((T)0);
         P.inv3.upload(inv3); P.im_off.upload(im_off);
         size_t nf = (size_t)P.total * P.ndim * nwave_;
@@ -1100,6 +1106,30 @@ private:
         P.veloc.alloc(nf); P.veloc.zero(stream_);
         if (sizeof(D) != sizeof(T)) { P.displ_elem.alloc(nf); P.displ_elem.zero(stream_); }
         if (COMP) { P.cd.alloc(nf); P.cd.zero(stream_); P.cv.alloc(nf); P.cv.zero(stream_); }
+    }
+    // per mode: what the point update does to it (MODE_*) and its point's 1 / M
+    void upload_mode_tables(PointDev &P, bool solid) {
+        std::vector<uint8_t> mf;
+        std::vector<T> mi;
+        mf.reserve(P.total); mi.reserve(P.total);
+        for (int p = 0; p < P.n; p++) {
+            const uint8_t fl = P.h_flags[p];
+            const int nr = P.h_nr[p], nu = P.h_nu[p];
+            for (int al = 0; al < nu; al++) {
+                uint8_t b = 0;
+                if (fl & (PT_MASS3D | PT_OCEAN)) b |= MODE_SKIP;
+                if (fl & PT_AXIAL) {
+                    if (solid) b |= al == 0 ? MODE_AXIS0 : al == 1 ? MODE_AXIS1 : MODE_ZERO;
+                    else if (al >= 1) b |= MODE_ZERO;
+                }
+                if (!solid && (fl & PT_SURFACE)) b |= MODE_ZERO;
+                if ((nr & 1) == 0 && al == nu - 1) b |= MODE_NYQUIST;
+                mf.push_back(b);
+                mi.push_back(P.h_inv1[p]);
+            }
+        }
+        P.mode_flags.upload(mf);
+        P.mode_inv.upload(mi);
     }
     // displacement as seen by the elements
     const C *elem_displ(const PointDev &P) const {
@@ -2143,8 +2173,8 @@ private:
                 post_launch();
             }
             PointArgs<T, D> a;
-            a.nmodes = P.total; a.ndim = P.ndim; a.solid = solid; a.mode_pt = P.mode_pt.p;
-            a.off = P.off.p; a.nr = P.nr.p; a.flags = P.flags.p; a.inv_mass1 = P.inv1.p;
+            a.nmodes = P.total; a.ndim = P.ndim; a.mode_flags = P.mode_flags.p; a.mode_inv = P.mode_inv.p;
+            a.mode_pt = P.mode_pt.p;
             a.stiff = P.stiff.p; a.accel = P.accel.p; a.displ = P.displ.p; a.veloc = P.veloc.p;
             a.cd = P.cd.p; a.cv = P.cv.p; a.displ_elem = P.displ_elem.p;
             if constexpr (sizeof(D) == sizeof(T)) {
@@ -2157,7 +2187,9 @@ private:
             a.mask = mask;
             a.nwave = nwave_;
             a.sponge = solid ? sg_s_.p : sg_f_.p;
-            int threads = POINT_BLOCK, blocks = (int)(((int64_t)P.total * nwave_ * P.ndim + threads - 1) / threads);
+            const int threads = POINT_BLOCK, modes = POINT_BLOCK / P.ndim;
+            const int wy = std::min(nwave_, 32768);
+            const dim3 blocks((unsigned)((P.total + modes - 1) / modes), (unsigned)wy, (unsigned)((nwave_ + wy - 1) / wy));
             Abc3D &g3 = solid ? sg3_s_ : sg3_f_;
             const bool press = !solid && ps_n_ && (mask & 2);
             if ((g3.n || press) && (mask & 2)) {

@@ -606,15 +606,21 @@ __global__ void ocean3d_kernel(const Ocean3DArgs<T> a) {
         for (int c = 0; c < 3; c++) f[al * 3 + c] = r2c_mode<T>(fr + (size_t)c * a.nr_max, nr, al, twc, tws);
 }
 
+// what the boundary conditions after assembly and the mass term do to one mode of one point
+// (AxialBoundary, FluidSurfaceBoundary, the Nyquist rule), formed once per mode on the host
+constexpr uint8_t MODE_SKIP = 1;    // Mass3D / ocean-load point: its own kernel does conditions and 1/M
+constexpr uint8_t MODE_AXIS0 = 2;   // solid axis, order 0: the horizontal components vanish
+constexpr uint8_t MODE_AXIS1 = 4;   // solid axis, order 1: horizontal components tied, vertical zero
+constexpr uint8_t MODE_ZERO = 8;    // higher orders on the axis, fluid surface
+constexpr uint8_t MODE_NYQUIST = 16;  // imaginary part dropped
+
 template <class T, class D>
 struct PointArgs {
     int nmodes;                  // sum nu
     int ndim;
-    int solid;
-    const int *mode_pt;          // [nmodes] owning point
-    const int *off, *nr;         // per point
-    const uint8_t *flags;
-    const T *inv_mass1;          // per point (1-D mass)
+    const uint8_t *mode_flags;   // [nmodes] MODE_*
+    const T *mode_inv;           // [nmodes] 1 / M of the owning point (1-D mass)
+    const int *mode_pt;          // [nmodes] owning point (sponge only)
     cx_t<T> *stiff;
     cx_t<T> *accel;
     cx_t<D> *displ, *veloc;
@@ -627,76 +633,77 @@ struct PointArgs {
     const T *sponge;             // [npoints] Kosloff gamma (0 = none) or null
 };
 
-// One thread per complex value of the point fields ([nwave][nmodes][ndim]), so that every field
-// is read and written in consecutive 8- / 16-byte words. The only condition that mixes the
-// components of a mode (the axial order-1 rule) reads the other component before the block's
-// barrier and every thread writes after it; blocks of POINT_BLOCK threads hold whole modes.
+// One thread per complex value of the point fields ([nmodes][ndim], a wavefield per (y, z)
+// block index), so that every field is read and written in consecutive 8- / 16-byte words. The only condition
+// that mixes the components of a mode (the axial order-1 rule) reads the other component before
+// the block's barrier and every thread writes after it; blocks of POINT_BLOCK threads hold whole
+// modes. Bound by HBM: 128 bytes per complex value in the mixed mode. The conditions and 1/M
+// come from per-mode tables, so that no load of a thread waits on another: all of them are in
+// flight at once (through the point of the mode, its offset, order, flags and mass followed one
+// another in three dependent rounds before the fields were asked for).
 constexpr int POINT_BLOCK = 288;   // 96 modes of 3 components, 9 warps
 template <class T, class D, bool COMP>
 __global__ void __launch_bounds__(POINT_BLOCK) point_update_kernel(const PointArgs<T, D> a) {
     const int nd = a.ndim;
-    const int64_t q64 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = q64 < (int64_t)a.nmodes * a.nwave * nd;
-    const size_t q = valid ? (size_t)q64 : 0;
-    const size_t m = nd == 3 ? q / 3 : q;              // mode of the batched fields
-    const int d = (int)(q - m * nd);
-    const int mm = a.nwave == 1 ? (int)m : (int)(m % (size_t)a.nmodes);
-    const int p = a.mode_pt[mm];
-    const int off = a.off[p], nr = a.nr[p], nu = nr / 2 + 1, al = mm - off;
-    const uint8_t fl = a.flags[p];
-    cx_t<T> f = valid ? a.stiff[q] : mk<T>(0, 0);
+    const int mb = nd == 3 ? (int)threadIdx.x / 3 : (int)threadIdx.x;
+    const int d = (int)threadIdx.x - mb * nd;
+    const int64_t m = (int64_t)blockIdx.x * (nd == 3 ? POINT_BLOCK / 3 : POINT_BLOCK) + mb;
+    const int w = (int)(blockIdx.z * gridDim.y + blockIdx.y);
+    const bool valid = m < a.nmodes && w < a.nwave;
+    const size_t mm = valid ? (size_t)m : 0;
+    const size_t q = valid ? ((size_t)w * a.nmodes + mm) * nd + d : 0;
+    const bool update = (a.mask & 4) != 0;
+    const uint8_t fl = a.mode_flags[mm];
+    const T inv = a.mode_inv[mm];
+    cx_t<T> f = a.stiff[q], acc = mk<T>(0, 0);
+    cx_t<D> v = mk<D>(0, 0), u = v;
+    cx_t<float> cv = mk<float>(0, 0), cd = cv;
+    if (update) {
+        acc = a.accel[q];
+        v = a.veloc[q];
+        u = a.displ[q];
+        if constexpr (COMP) { cv = a.cv[q]; cd = a.cd[q]; }
+    }
     // the axial rule of order 1 (solid): both horizontal components of the mode
-    const bool mix = valid && (a.mask & 1) && a.solid && (fl & PT_AXIAL) && al == 1 && d < 2 &&
-                     !(fl & (PT_MASS3D | PT_OCEAN));
+    const bool mix = (a.mask & 1) && (fl & MODE_AXIS1) && d < 2 && !(fl & MODE_SKIP);
     cx_t<T> g0 = f, g1 = f;
     if (mix) {
-        g0 = a.stiff[m * 3];
-        g1 = a.stiff[m * 3 + 1];
+        g0 = a.stiff[q - d];
+        g1 = a.stiff[q - d + 1];
     }
     __syncthreads();
     if (!valid) return;
-    if (!(fl & (PT_MASS3D | PT_OCEAN))) {
+    if (!(fl & MODE_SKIP)) {
         if (a.mask & 1) {
-            // point_bc for one component (AxialBoundary::apply, the fluid surface, the Nyquist
-            // imaginary parts)
+            // point_bc for one component
             const T half = (T)0.5;
-            if (fl & PT_AXIAL) {
-                if (a.solid) {
-                    if (al == 0) {
-                        if (d < 2) f = mk<T>(0, 0);
-                    } else if (al == 1) {
-                        const cx_t<T> t = mk<T>((g0.x + g1.y) * half, (g0.y - g1.x) * half);
-                        f = d == 0 ? t : d == 1 ? mk<T>(-t.y, t.x) : mk<T>(0, 0);
-                    } else {
-                        f = mk<T>(0, 0);
-                    }
-                } else if (al >= 1) {
-                    f = mk<T>(0, 0);
-                }
+            if (fl & MODE_AXIS0) {
+                if (d < 2) f = mk<T>(0, 0);
+            } else if (fl & MODE_AXIS1) {
+                const cx_t<T> t = mk<T>((g0.x + g1.y) * half, (g0.y - g1.x) * half);
+                f = d == 0 ? t : d == 1 ? mk<T>(-t.y, t.x) : mk<T>(0, 0);
             }
-            if (!a.solid && (fl & PT_SURFACE)) f = mk<T>(0, 0);
-            if ((nr & 1) == 0 && al == nu - 1) f.y = 0;
+            if (fl & MODE_ZERO) f = mk<T>(0, 0);
+            if (fl & MODE_NYQUIST) f.y = 0;
         }
-        if (a.mask & 2) f = cscale(f, a.inv_mass1[p]);
+        if (a.mask & 2) f = cscale(f, inv);
     }
     if ((a.mask & 2) && a.sponge) {
         // Sponge::apply (ABC/Sponge.hpp:74-98), 1-D gamma, on the acceleration
-        const T g = a.sponge[p];
+        const T g = a.sponge[a.mode_pt[mm]];
         if (g != (T)0) {
             const T two = 2;
-            const cx_t<T> v = mk<T>((T)a.veloc[q].x, (T)a.veloc[q].y);
-            const cx_t<T> u = mk<T>((T)a.displ[q].x, (T)a.displ[q].y);
-            f = csub(f, cadd(cscale(v, two * g), cscale(u, g * g)));
+            if (!update) { v = a.veloc[q]; u = a.displ[q]; }
+            const cx_t<T> vt = mk<T>((T)v.x, (T)v.y), ut = mk<T>((T)u.x, (T)u.y);
+            f = csub(f, cadd(cscale(vt, two * g), cscale(ut, g * g)));
         }
     }
-    if (!(a.mask & 4)) {
+    if (!update) {
         // stages without the update: the result stays in the stiffness field, as
         // computeStiffToAccel works in place on mStiff
         a.stiff[q] = f;
         return;
     }
-    const cx_t<T> acc = a.accel[q];
-    cx_t<D> v = a.veloc[q], u = a.displ[q];
     if constexpr (sizeof(D) == sizeof(T)) {
         // NewmarkTimeScheme::update in the working precision
         v.x += a.half_dt * (acc.x + f.x);
@@ -707,7 +714,6 @@ __global__ void __launch_bounds__(POINT_BLOCK) point_update_kernel(const PointAr
         const D dvx = a.half_dt * ((D)acc.x + (D)f.x);
         const D dvy = a.half_dt * ((D)acc.y + (D)f.y);
         if constexpr (COMP) {
-            cx_t<float> cv = a.cv[q], cd = a.cd[q];
             D y = dvx - (D)cv.x, t = v.x + y; cv.x = (float)((t - v.x) - y); v.x = t;
             y = dvy - (D)cv.y; t = v.y + y; cv.y = (float)((t - v.y) - y); v.y = t;
             const D dux = a.dt * v.x + a.half_dt_dt * (D)f.x;

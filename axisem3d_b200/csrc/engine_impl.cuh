@@ -17,6 +17,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <functional>
 #include <map>
 #include <mutex>
 #include <numeric>
@@ -169,6 +170,9 @@ public:
         if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
         if (ev0_) cudaEventDestroy(ev0_);
         if (ev1_) cudaEventDestroy(ev1_);
+        if (fork_ev_) cudaEventDestroy(fork_ev_);
+        for (cudaEvent_t e : join_ev_) cudaEventDestroy(e);
+        for (cudaStream_t q : side_) cudaStreamDestroy(q);
         if (own_stream_) cudaStreamDestroy(own_stream_);
     }
 
@@ -226,6 +230,7 @@ public:
         nonfinite_.zero(stream_);
         AXG_CUDA(cudaEventCreate(&ev0_));
         AXG_CUDA(cudaEventCreate(&ev1_));
+        build_side_streams();
         AXG_CUDA(cudaStreamSynchronize(stream_));
         finalized_ = true;
     }
@@ -251,9 +256,7 @@ public:
         if (tstep < 0) throw Error(AXG_E_ARG, "Domain::recordOutput || negative time step.");
         ensure_capacity(tstep + 1);
         set_step(tstep);
-        launch_stations();
-        launch_element_record();
-        launch_scan();
+        launch_records();
     }
 
     void run(int nsteps, bool graph) override {
@@ -261,6 +264,7 @@ public:
         if (nsteps <= 0) return;
         ensure_capacity(step_ + nsteps);
         set_step(step_);
+        dev_step_ = -1;   // the steps advance it; known again when all of them are queued
         if (timing_) {
             for (int i = 0; i < nsteps; i++) {
                 launch_step();
@@ -280,6 +284,7 @@ public:
             for (int i = 0; i < nsteps; i++) launch_step();
         }
         step_ += nsteps;
+        dev_step_ = step_;
         if (cfg_.stability_interval > 0) check_finite();
     }
     int step() const override { return step_; }
@@ -485,6 +490,7 @@ public:
     }
     void set_stream(void *s) override {
         stream_ = s ? (cudaStream_t)s : own_stream_;
+        dev_step_ = -1;   // set again in the new stream's order
         if (graph_exec_) { cudaGraphExecDestroy(graph_exec_); graph_exec_ = nullptr; }
     }
     void set_team_override(int cls, int team) override {
@@ -566,6 +572,7 @@ public:
             copy_fields_in(c);
             step_ = ck_step0_ + c * ck_interval_;
             set_step(step_);
+            dev_step_ = -1;
             // recompute the segment, keeping u_n and a_n (the forward step's graph, which reads
             // the step from the device counter set above)
             if (!cfg_.plain && !graph_exec_) capture();
@@ -714,7 +721,12 @@ public:
             throw Error(AXG_E_ARG, std::string(who) + "the model's SLS state (" + std::to_string(need_bytes) +
                                        " bytes) exceeds the fixed scratch of " + std::to_string(cap) + " bytes.");
         if (need_bytes) AXG_CUDA(cudaMemsetAsync(scratch, 0, need_bytes, stream_));
-        for (auto &bp : sb_) {
+        std::vector<Branch> br;
+        std::vector<SolidBucket *> bs;
+        for (auto &bp : sb_) bs.push_back(bp.get());
+        if (!cfg_.deterministic)
+            std::stable_sort(bs.begin(), bs.end(), [](SolidBucket *x, SolidBucket *y) { return x->bytes > y->bytes; });
+        for (SolidBucket *bp : bs) br.push_back([=] {
             SolidBucket &b = *bp;
             SolidArgs<T, AT> a;
             a.n_elem = b.n; a.nr = b.nr.p; a.pts = b.pts.p; a.axial = b.axial.p;
@@ -733,8 +745,8 @@ public:
             a.fstride = 0;
             a.sstride = 0;
             launch_solid_args(b, a);
-        }
-        for (auto &bp : fb_) {
+        });
+        for (auto &fp : fb_) br.push_back([=, bp = fp.get()] {
             FluidBucket &b = *bp;
             FluidArgs<T> a;
             a.n_elem = b.n; a.nr = b.nr.p; a.pts = b.pts.p; a.axial = b.axial.p; a.geom = b.geom.p;
@@ -746,10 +758,15 @@ public:
             a.fstride = 0;
             a.x = b.xpool.p; a.x_off = b.xoff.p; a.x3d = b.x3d.p; a.trig = b.trig.p;
             int blocks = (b.n + b.tpc - 1) / b.tpc;
-            b.kernel<<<blocks, b.team * b.tpc, b.tpc * b.team_bytes, stream_>>>(a, b.nr_max, b.tpc,
+            b.kernel<<<blocks, b.team * b.tpc, b.tpc * b.team_bytes, ls()>>>(a, b.nr_max, b.tpc,
                                                                               b.team_bytes);
             post_launch();
-        }
+        });
+        // one after another where the sums must come in one order
+        if (cfg_.deterministic)
+            for (auto &f : br) f();
+        else
+            run_branches(br);
     }
     int device() const override { return cfg_.device; }
 
@@ -992,10 +1009,17 @@ private:
     void need() const {
         if (!finalized_) throw Error(AXG_E_STATE, "Engine::step || axg_finalize not called.");
     }
+    // the device step counter, set by a one-thread kernel when it does not hold the step already
+    // (a copy from the host and its synchronisation took two round trips of every hook-driven step)
     void set_step(int tstep) {
-        tstep_host_ = tstep;
-        AXG_CUDA(cudaMemcpyAsync(step_dev_.p, &tstep_host_, sizeof(int), cudaMemcpyHostToDevice, stream_));
-        AXG_CUDA(cudaStreamSynchronize(stream_));
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        AXG_CUDA(cudaStreamIsCapturing(stream_, &cap));
+        if (cap != cudaStreamCaptureStatusNone)
+            throw Error(AXG_E_CUDA, "Engine::set_step || the time step cannot be set while the stream is capturing.");
+        if (dev_step_ == tstep) return;
+        set_step_kernel<T><<<1, 1, 0, stream_>>>(step_dev_.p, tstep);
+        AXG_CUDA(cudaGetLastError());
+        dev_step_ = tstep;
     }
     void check_finite() {
         int flag = 0;
@@ -1687,7 +1711,7 @@ private:
                 a.first = solid ? cls_first_.p : clf_first_.p;
                 a.c = solid ? cls_c_.p : clf_c_.p; a.veloc = P.veloc.p; a.stiff = P.stiff.p;
                 a.nwave = nwave_; a.fstride = (size_t)P.total * P.ndim;
-                clayton_kernel<T, D><<<(n * 32 + 255) / 256, 256, 0, stream_>>>(a);
+                clayton_kernel<T, D><<<(n * 32 + 255) / 256, 256, 0, ls()>>>(a);
                 post_launch();
             }
             Abc3D &c3 = solid ? cl3_s_ : cl3_f_;
@@ -1699,7 +1723,7 @@ private:
                 a.fstride = (size_t)P.total * P.ndim;
                 const int wpb = 4;
                 clayton3d_kernel<T, D><<<(c3.n * nwave_ + wpb - 1) / wpb, 32 * wpb,
-                                         (size_t)wpb * 6 * P.nr_max * sizeof(T), stream_>>>(a);
+                                         (size_t)wpb * 6 * P.nr_max * sizeof(T), ls()>>>(a);
                 post_launch();
             }
         }
@@ -1746,7 +1770,7 @@ private:
             a.step = step_dev_.p;
             a.h2p = S.h2p.p; a.h2pp = S.h2pp.p; a.cnt = S.cnt.p; a.key = S.key.p; a.nu1 = S.nu1.p;
             const int m = S.n * P.ndim;
-            scan_kernel<T, D><<<(m + 255) / 256, 256, 0, stream_>>>(a);
+            scan_kernel<T, D><<<(m + 255) / 256, 256, 0, ls()>>>(a);
             post_launch();
         }
     }
@@ -1790,7 +1814,7 @@ private:
         a.stiff = P.stiff.p; a.nr_max = P.nr_max; a.nwave = nwave_; a.fstride = (size_t)P.total * P.ndim;
         const int wpb = 4;
         sponge3d_kernel<T, D><<<(g.n * nwave_ + wpb - 1) / wpb, 32 * wpb, (size_t)wpb * 3 * P.nr_max * sizeof(T),
-                                stream_>>>(a);
+                                ls()>>>(a);
         post_launch();
     }
 
@@ -1964,7 +1988,7 @@ private:
             a.e_nr = e_nr_.p; a.e_pts = e_pts_.p; a.e_axial = e_axial_.p; a.e_geom = e_geom_.p;
             a.pt_off = sp_.off.p; a.pt_nu = sp_.nu.p; a.stiff = sp_.stiff.p; a.gmat = gmat_.p;
             a.wave = ms_wave_.p; a.fstride = (size_t)sp_.total * 3;
-            moment_source_kernel<T><<<ms_n_, 128, 0, stream_>>>(a);
+            moment_source_kernel<T><<<ms_n_, 128, 0, ls()>>>(a);
             post_launch();
         }
         if (fs_n_) {
@@ -1973,7 +1997,7 @@ private:
             a.pattern = fs_pat_.p; a.stf = fs_stf_.p; a.stf_steps = stf_cap_; a.step = step_dev_.p;
             a.e_pts = e_pts_.p; a.pt_off = sp_.off.p; a.pt_nu = sp_.nu.p; a.stiff = sp_.stiff.p;
             a.wave = fs_wave_.p; a.fstride = (size_t)sp_.total * 3;
-            force_source_kernel<T><<<fs_n_, 128, 0, stream_>>>(a);
+            force_source_kernel<T><<<fs_n_, 128, 0, ls()>>>(a);
             post_launch();
         }
     }
@@ -1986,17 +2010,94 @@ private:
         a.pattern = ps_pat_.p; a.stf = ps_stf_.p; a.stf_steps = stf_cap_; a.step = step_dev_.p;
         a.e_pts = fe_pts_.p; a.pt_off = fp_.off.p; a.pt_nu = fp_.nu.p; a.stiff = fp_.stiff.p;
         a.wave = ps_wave_.p; a.fstride = (size_t)fp_.total;
-        pressure_source_kernel<T><<<ps_n_, 128, 0, stream_>>>(a);
+        pressure_source_kernel<T><<<ps_n_, 128, 0, ls()>>>(a);
         post_launch();
+    }
+
+    // the side streams of run_branches, as many as the step has branches beyond the first (at
+    // most 7); made with the handle, since a branch may run while a caller's stream is capturing
+    void build_side_streams() {
+        size_t n = sb_.size() + fb_.size() + (ms_n_ || fs_n_) + 1;
+        if (cfg_.plain) n = 1;
+        n = std::min<size_t>(n - 1, 7);
+        AXG_CUDA(cudaEventCreateWithFlags(&fork_ev_, cudaEventDisableTiming));
+        for (size_t i = 0; i < n; i++) {
+            cudaStream_t q = nullptr;
+            AXG_CUDA(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking));
+            side_.push_back(q);
+            cudaEvent_t e = nullptr;
+            AXG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+            join_ev_.push_back(e);
+        }
+    }
+    // Independent launches of a step. Each branch is a chain of launches; the first stays on the
+    // handle's stream, the others go round-robin to side streams that start after what is queued
+    // so far and are joined before whatever follows (graph edges under capture). The buckets of a
+    // mesh with uneven nr, the sources and the stations are mostly too few blocks to fill the GPU
+    // on their own, and their last waves overlap this way. The plain method keeps one stream.
+    using Branch = std::function<void()>;
+    void run_branches(std::vector<Branch> &br) {
+        const size_t nside = cfg_.plain || br.empty() ? 0 : std::min(br.size() - 1, side_.size());
+        if (nside == 0) {
+            for (auto &f : br) f();
+            return;
+        }
+        struct Reset {
+            cudaStream_t &s;
+            ~Reset() { s = nullptr; }
+        } reset{branch_};
+        AXG_CUDA(cudaEventRecord(fork_ev_, stream_));
+        for (size_t i = 0; i < nside; i++) AXG_CUDA(cudaStreamWaitEvent(side_[i], fork_ev_, 0));
+        for (size_t k = 0; k < br.size(); k++) {
+            const size_t i = k % (nside + 1);
+            branch_ = i == 0 ? nullptr : side_[i - 1];
+            br[k]();
+        }
+        branch_ = nullptr;
+        for (size_t i = 0; i < nside; i++) {
+            AXG_CUDA(cudaEventRecord(join_ev_[i], side_[i]));
+            AXG_CUDA(cudaStreamWaitEvent(stream_, join_ev_[i], 0));
+        }
+    }
+    cudaStream_t ls() const { return branch_ ? branch_ : stream_; }
+
+    // the solid buckets (of one part, or all with part < 0) as branches, the most bytes first;
+    // deterministic assembly needs the colours one after another: one branch
+    void solid_branches(std::vector<Branch> &br, int part) {
+        std::vector<SolidBucket *> bs;
+        for (auto &bp : sb_)
+            if (part < 0 || bp->part == part) bs.push_back(bp.get());
+        if (cfg_.deterministic) {
+            if (!bs.empty()) br.push_back([this, bs] { for (SolidBucket *b : bs) launch_solid_bucket(*b); });
+            return;
+        }
+        std::stable_sort(bs.begin(), bs.end(), [](SolidBucket *x, SolidBucket *y) { return x->bytes > y->bytes; });
+        for (SolidBucket *b : bs) br.push_back([this, b] { launch_solid_bucket(*b); });
+    }
+    void fluid_branches(std::vector<Branch> &br, int part) {
+        std::vector<FluidBucket *> bs;
+        for (auto &bp : fb_)
+            if (part < 0 || bp->part == part) bs.push_back(bp.get());
+        if (cfg_.deterministic) {
+            if (!bs.empty()) br.push_back([this, bs] { for (FluidBucket *b : bs) launch_fluid_bucket(*b); });
+            return;
+        }
+        for (FluidBucket *b : bs) br.push_back([this, b] { launch_fluid_bucket(*b); });
     }
 
     // every bucket (part < 0) or the buckets of one element part
     void launch_stiffness(int part = -1) {
-        if (timing_) AXG_CUDA(cudaEventRecord(ev0_, stream_));
-        for (auto &bp : sb_)
-            if (part < 0 || bp->part == part) launch_solid_bucket(*bp);
-        if (timing_) AXG_CUDA(cudaEventRecord(ev1_, stream_));
-        launch_fluid(part);
+        std::vector<Branch> br;
+        solid_branches(br, part);
+        if (timing_) {
+            // the events bracket the solid buckets only
+            AXG_CUDA(cudaEventRecord(ev0_, stream_));
+            run_branches(br);
+            AXG_CUDA(cudaEventRecord(ev1_, stream_));
+            br.clear();
+        }
+        fluid_branches(br, part);
+        run_branches(br);
     }
 
     void launch_solid_bucket(SolidBucket &b) {
@@ -2026,22 +2127,20 @@ private:
         if (b.prt) {
             PrtArgs<T, AT> pa;
             pa.s = a; pa.x = b.xpool.p; pa.x_off = b.xoff.p; pa.x3d = b.x3d.p;
-            b.pkernel<<<b.grid, b.team * b.tpc, b.tpc * b.team_bytes, stream_>>>(pa, b.nr_max, b.qc, b.tpc,
+            b.pkernel<<<b.grid, b.team * b.tpc, b.tpc * b.team_bytes, ls()>>>(pa, b.nr_max, b.qc, b.tpc,
                                                                                b.team_bytes);
         } else {
             SolidArgs<T, AT> af = a;
             af.fft_min_nr = b.fft ? AXG_FFT_MIN_NR : 0;
             af.prefetch_ahead = b.ahead;
-            b.kernel<<<b.grid, b.team * b.tpc, b.tpc * b.team_bytes, stream_>>>(af, b.nr_max, b.qc, b.mt, b.tpc,
+            b.kernel<<<b.grid, b.team * b.tpc, b.tpc * b.team_bytes, ls()>>>(af, b.nr_max, b.qc, b.mt, b.tpc,
                                                                               b.team_bytes);
         }
         post_launch();
     }
 
-    void launch_fluid(int part = -1) {
-        for (auto &bp : fb_) {
-            FluidBucket &b = *bp;
-            if (part >= 0 && b.part != part) continue;
+    void launch_fluid_bucket(FluidBucket &b) {
+        {
             FluidArgs<T> a;
             a.n_elem = b.n; a.nr = b.nr.p; a.pts = b.pts.p; a.axial = b.axial.p; a.geom = b.geom.p;
             a.K = b.K.p; a.K_off = b.K_off.p; a.pt_off = fp_.off.p; a.pt_nu = fp_.nu.p;
@@ -2051,7 +2150,7 @@ private:
             a.fstride = (size_t)fp_.total;
             a.x = b.xpool.p; a.x_off = b.xoff.p; a.x3d = b.x3d.p; a.trig = b.trig.p;
             int blocks = (b.n + b.tpc - 1) / b.tpc;
-            b.kernel<<<blocks, b.team * b.tpc, b.tpc * b.team_bytes, stream_>>>(a, b.nr_max, b.tpc,
+            b.kernel<<<blocks, b.team * b.tpc, b.tpc * b.team_bytes, ls()>>>(a, b.nr_max, b.tpc,
                                                                               b.team_bytes);
             post_launch();
         }
@@ -2085,7 +2184,7 @@ private:
             a.s_stride = (size_t)sp_.total * 3; a.f_stride = (size_t)fp_.total;
             const int wpb = 4;
             solid_fluid3d_kernel<T><<<(cp3_n_ * nwave_ + wpb - 1) / wpb, 32 * wpb,
-                                      (size_t)wpb * 4 * cp3_nr_max_ * sizeof(T), stream_>>>(a);
+                                      (size_t)wpb * 4 * cp3_nr_max_ * sizeof(T), ls()>>>(a);
             post_launch();
         }
         if (!cp_n_) return;
@@ -2096,7 +2195,7 @@ private:
         a.s_displ = elem_displ(sp_); a.s_stiff = sp_.stiff.p; a.f_stiff = fp_.stiff.p;
         a.nwave = nwave_; a.s_stride = (size_t)sp_.total * 3; a.f_stride = (size_t)fp_.total;
         int threads = 256, blocks = (cp_n_ * 32 + threads - 1) / threads;
-        solid_fluid_kernel<T><<<blocks, threads, 0, stream_>>>(a);
+        solid_fluid_kernel<T><<<blocks, threads, 0, ls()>>>(a);
         post_launch();
     }
 
@@ -2110,7 +2209,7 @@ private:
         a.nwave = nwave_; a.fstride = (size_t)sp_.total * 3;
         const int threads = 128;                          // four stations per block
         const int blocks = (int)(((size_t)st_n_ * nwave_ * 32 + threads - 1) / threads);
-        station_kernel<T><<<blocks, threads, 0, stream_>>>(a);
+        station_kernel<T><<<blocks, threads, 0, ls()>>>(a);
         post_launch();
         if (model_.st.gradient) {
             StationGradArgs<T> g;
@@ -2119,7 +2218,7 @@ private:
             g.gmat = gmat_.p; g.pt_off = sp_.off.p; g.pt_nu = sp_.nu.p; g.displ = elem_displ(sp_);
             g.out = seis_grad_.p; g.interval = st_interval_; g.max_rec = seis_cap_; g.step = step_dev_.p;
             g.nwave = nwave_; g.fstride = (size_t)sp_.total * 3;
-            station_grad_kernel<T><<<blocks, threads, 0, stream_>>>(g);
+            station_grad_kernel<T><<<blocks, threads, 0, ls()>>>(g);
             post_launch();
         }
     }
@@ -2134,14 +2233,22 @@ private:
         a.step = step_dev_.p; a.nwave = nwave_; a.fstride = (size_t)sp_.total * 3;
         const int threads = 256;                          // eight entries per block
         const int blocks = (int)(((size_t)er_n_ * nwave_ * 32 + threads - 1) / threads);
-        element_record_kernel<T><<<blocks, threads, 0, stream_>>>(a);
+        element_record_kernel<T><<<blocks, threads, 0, ls()>>>(a);
         post_launch();
     }
 
-    void launch_points(int mask) {
-        for (int solid = 1; solid >= 0; solid--) {
+    void launch_points(int mask, bool advance = false) {
+        // the last point set's update (the one that pressure sources precede) advances the step
+        const int last = fp_.n ? 0 : 1;
+        std::vector<Branch> br;
+        for (int solid = 1; solid >= 0; solid--)
+            if ((solid ? sp_ : fp_).n) br.push_back([=] { launch_point_set(solid, mask, advance && solid == last); });
+        run_branches(br);
+    }
+
+    void launch_point_set(int solid, int mask, bool advance) {
+        {
             PointDev &P = solid ? sp_ : fp_;
-            if (!P.n) continue;
             if (P.n3d && (mask & 3)) {
                 Mass3DArgs<T> a;
                 a.n = P.n3d; a.pt = P.pt3d.p; a.nr = P.nr.p; a.off = P.off.p; a.flags = P.flags.p;
@@ -2150,7 +2257,7 @@ private:
                 a.nwave = nwave_; a.fstride = (size_t)P.total * P.ndim;
                 a.mask = mask;
                 int wpb = 4;
-                mass3d_kernel<T><<<(P.n3d * nwave_ + wpb - 1) / wpb, 32 * wpb, wpb * P.nr_max * sizeof(T), stream_>>>(a);
+                mass3d_kernel<T><<<(P.n3d * nwave_ + wpb - 1) / wpb, 32 * wpb, wpb * P.nr_max * sizeof(T), ls()>>>(a);
                 post_launch();
             }
             if (solid && ocean3_n_ && (mask & 3)) {
@@ -2161,7 +2268,7 @@ private:
                 o.fstride = (size_t)P.total * P.ndim; o.mask = mask;
                 const int wpb = 4;
                 ocean3d_kernel<T><<<(ocean3_n_ * nwave_ + wpb - 1) / wpb, 32 * wpb,
-                                    (size_t)wpb * 3 * P.nr_max * sizeof(T), stream_>>>(o);
+                                    (size_t)wpb * 3 * P.nr_max * sizeof(T), ls()>>>(o);
                 post_launch();
             }
             if (solid && ocean_n_ && (mask & 3)) {
@@ -2169,7 +2276,7 @@ private:
                 o.n = ocean_n_; o.pt = ocean_pt_.p; o.c = ocean_c_.p; o.nr = P.nr.p; o.off = P.off.p;
                 o.flags = P.flags.p; o.stiff = P.stiff.p; o.nwave = nwave_;
                 o.fstride = (size_t)P.total * P.ndim; o.mask = mask;
-                ocean_mass_kernel<T><<<(ocean_n_ * nwave_ * 32 + 255) / 256, 256, 0, stream_>>>(o);
+                ocean_mass_kernel<T><<<(ocean_n_ * nwave_ * 32 + 255) / 256, 256, 0, ls()>>>(o);
                 post_launch();
             }
             PointArgs<T, D> a;
@@ -2184,6 +2291,7 @@ private:
                 a.dt = cfg_.dt; a.half_dt = .5 * cfg_.dt; a.half_dt_dt = .5 * cfg_.dt * cfg_.dt;
             }
             a.nonfinite = nonfinite_.p;
+            a.step = nullptr;
             a.mask = mask;
             a.nwave = nwave_;
             a.sponge = solid ? sg_s_.p : sg_f_.p;
@@ -2196,29 +2304,53 @@ private:
                 // a 3-D sponge and fluid pressure sources act on the acceleration between
                 // 1/M and the update
                 a.mask = mask & 3;
-                point_update_kernel<T, D, COMP><<<blocks, threads, 0, stream_>>>(a);
+                point_update_kernel<T, D, COMP><<<blocks, threads, 0, ls()>>>(a);
                 post_launch();
                 if (g3.n) launch_sponge3d(P, g3);
                 if (press) launch_pressure_sources();
-                if (!(mask & 4)) continue;
+                if (!(mask & 4)) return;
                 a.mask = 4;
             }
-            point_update_kernel<T, D, COMP><<<blocks, threads, 0, stream_>>>(a);
+            a.step = advance ? step_dev_.p : nullptr;
+            point_update_kernel<T, D, COMP><<<blocks, threads, 0, ls()>>>(a);
             post_launch();
         }
     }
 
+    // one time step: the element kernels, the sources (atomic adds to the same stiffness) and the
+    // recordings (which read the displacement) side by side, then the couplings that read what
+    // they summed, then the points
     void launch_step() {
-        launch_sources();
-        launch_stiffness();
+        if (timing_ || cfg_.plain) {
+            launch_sources();
+            launch_stiffness();
+            launch_records();
+        } else {
+            std::vector<Branch> br;
+            if (cfg_.deterministic) {
+                std::vector<Branch> solid;
+                solid_branches(solid, -1);
+                br.push_back([this, solid] {
+                    launch_sources();
+                    for (auto &f : solid) f();
+                });
+                fluid_branches(br, -1);
+            } else {
+                solid_branches(br, -1);
+                fluid_branches(br, -1);
+                if (ms_n_ || fs_n_) br.push_back([this] { launch_sources(); });
+            }
+            if (st_n_ || er_n_ || model_.scan.enabled) br.push_back([this] { launch_records(); });
+            run_branches(br);
+        }
         launch_clayton();
         launch_coupling();
+        launch_points(7, true);
+    }
+    void launch_records() {
         launch_stations();
         launch_element_record();
         launch_scan();
-        launch_points(7);
-        advance_step_kernel<T><<<1, 1, 0, stream_>>>(step_dev_.p);
-        post_launch();
     }
 
     void post_launch() {
@@ -2250,8 +2382,12 @@ private:
     HostModel model_;
     cudaDeviceProp prop_;
     cudaStream_t own_stream_ = nullptr, stream_ = nullptr;
+    cudaStream_t branch_ = nullptr;       // the side stream that launches go to, or null: stream_
+    std::vector<cudaStream_t> side_;
+    std::vector<cudaEvent_t> join_ev_;
+    cudaEvent_t fork_ev_ = nullptr;
     bool finalized_ = false;
-    int step_ = 0, tstep_host_ = 0;
+    int step_ = 0, dev_step_ = -1;   // dev_step_: what the device counter holds, -1 = unknown
     int64_t launches_ = 0, kernels_per_step_ = 0;
     bool timing_ = false;
     double time_ms_ = 0;

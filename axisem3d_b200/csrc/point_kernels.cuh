@@ -628,6 +628,7 @@ struct PointArgs {
     cx_t<T> *displ_elem;         // float copy of d for elements (MIXED) or null
     D dt, half_dt, half_dt_dt;
     int *nonfinite;
+    int *step;                   // device step counter to advance, or null
     int mask;                    // 1 = BC after assembly, 2 = 1/M, 4 = Newmark
     int nwave;                   // wavefields; fields are [nwave][nmodes][ndim]
     const T *sponge;             // [npoints] Kosloff gamma (0 = none) or null
@@ -734,6 +735,7 @@ __global__ void __launch_bounds__(POINT_BLOCK) point_update_kernel(const PointAr
     a.accel[q] = f;
     a.stiff[q] = mk<T>(0, 0);
     if (!(isfinite(u.x) && isfinite(u.y))) atomicOr(a.nonfinite, 1);
+    if (q == 0 && a.step) *a.step += 1;
 }
 
 // ------------------------------------------------------------------ sources ---
@@ -1157,7 +1159,7 @@ __global__ void narrow_kernel(const cx_t<D> *src, cx_t<T> *dst, size_t n) {
 }
 
 template <class T>
-__global__ void advance_step_kernel(int *step) { *step += 1; }
+__global__ void set_step_kernel(int *step, int value) { *step = value; }
 
 
 // ------------------------------------------------- boundary-stiffness exchange ---

@@ -127,7 +127,6 @@ class Engine final : public EngineBase {
         int part = 0;   // element part (axg_set_element_parts)
         int mt = 1;   // Fourier modes per tile of the gather / gradient and the quadrature
         int fft = 0;  // 3-D elements of nr >= AXG_FFT_MIN_NR take the slice FFTs
-        int ahead = 0;   // L2 prefetch distance in elements (AXG_PREFETCH_AHEAD waves), 0 = off
         size_t team_bytes;
         DBuf<int> nr, pts;
         DBuf<uint8_t> axial;
@@ -135,6 +134,12 @@ class Engine final : public EngineBase {
         DBuf<int64_t> mod_off, att_off, state_off;
         double bytes = 0, flops = 0;
         void (*kernel)(const SolidArgs<T, AT>, int, int, int, int, size_t) = nullptr;
+        // elements without 3-D properties: their own kernel over tiles of modes
+        void (*kernel1d)(const SolidArgs<T, AT>, int) = nullptr;
+        std::vector<int> h_nr;
+        std::vector<uint8_t> h_axial;
+        DBuf<int4> tiles;
+        DBuf<int2> tab;
         // particle relabelling (undulated geometry): its own kernel and factors
         int prt = 0;
         DBuf<T> xpool;
@@ -1310,6 +1315,9 @@ private:
             b->bytes = bytes;
             b->flops = flops;
             b->nr.upload(nr); b->pts.upload(pts); b->axial.upload(ax);
+            std::vector<int2> tab((size_t)b->n * 25);
+            for (size_t i = 0; i < tab.size(); i++) tab[i] = make_int2(sp_.h_off[pts[i]], sp_.h_nu[pts[i]]);
+            b->tab.upload(tab);
             b->geom.upload(geom);
             if (trig.empty()) trig.push_back((T)0);
             b->trig.upload(trig);
@@ -1326,7 +1334,13 @@ private:
                 // hold an nr of at least AXG_FFT_MIN_NR (the plain method keeps the direct sums)
                 const bool reg_path = b->att == ATT_NONE || cfg_.nsls == 3 || cfg_.nsls == 5;
                 b->fft = (!cfg_.plain && b->is3d && reg_path && AXG_FFT_MIN_NR > 0 && b->nr_max >= AXG_FFT_MIN_NR) ? 1 : 0;
-                b->kernel = pick_solid<T, AT>(b->rheo, b->att, b->is3d, b->rtz, cfg_.nsls, b->fft != 0);
+                if (b->is3d) {
+                    b->kernel = pick_solid<T, AT>(b->rheo, b->att, b->rtz, cfg_.nsls, b->fft != 0);
+                } else {
+                    b->kernel1d = pick_solid_1d<T, AT>(b->rheo, b->att, b->rtz, cfg_.nsls);
+                    b->h_nr = nr;
+                    b->h_axial = ax;
+                }
             }
             configure_bucket(*b);
             sb_.push_back(std::move(b));
@@ -1340,7 +1354,42 @@ private:
 #ifndef AXG_QC_FOR_TWO_CTAS
 #define AXG_QC_FOR_TWO_CTAS 1
 #endif
+    // Blocks of a 1-D bucket: every element's modes in equal tiles of at most `cap`, one thread per
+    // (mode, point). Five modes (128 threads, 125 of them busy) by default: smaller tiles repeat
+    // the element's operands, larger ones leave fewer blocks per SM to hide each other's latency.
+    // A team size that the caller or the autotuner sets gives the tile its threads hold.
+    void configure_1d(SolidBucket &b, int team_req) {
+        const int team = team_req ? team_req : (cfg_.plain ? 256 : team_override_[b.cls]);
+        const int cap = team ? team / 25 : 5;
+        std::vector<int4> tiles;
+        int mt = 1;
+        for (int e = 0; e < b.n; e++) {
+            const int nu = b.h_nr[e] / 2 + 1, nt = (nu + cap - 1) / cap;
+            for (int t = 0, t0 = 0; t < nt; t++) {
+                const int m = (nu - t0 + nt - t - 1) / (nt - t);
+                tiles.push_back(make_int4(e, t0, m, nu | (b.h_axial[e] ? 1 << 30 : 0)));
+                mt = std::max(mt, m);
+                t0 += m;
+            }
+        }
+        b.tiles.upload(tiles);
+        b.mt = mt;
+        b.qc = 25;
+        b.tpc = 1;
+        b.team = team ? team : (25 * mt + 31) / 32 * 32;
+        b.team_bytes = b.att == ATT_CG4 ? tile_1d<T, AT, ATT_CG4>(mt).total : tile_1d<T, AT, ATT_NONE>(mt).total;
+        b.grid = (int)tiles.size();
+        raise_smem_limit((const void *)b.kernel1d, b.team_bytes);
+    }
+    // wavefields of a batch on (y, z) of the grid: split over blocks while the elements alone do
+    // not fill the GPU several times over (each split loads the element's operands again)
+    dim3 wave_grid(int blocks) const {
+        const int want = std::max(1, prop_.multiProcessorCount * 16 / std::max(blocks, 1));
+        return dim3((unsigned)blocks, (unsigned)std::min({nwave_, want, 65535}), 1);
+    }
+
     void configure_bucket(SolidBucket &b, int team_req = 0) {
+        if (b.kernel1d) { configure_1d(b, team_req); return; }
         int team = team_req ? team_req
                             : (cfg_.plain ? 256 : (team_override_[b.cls] ? team_override_[b.cls] : default_team(b.cls)));
         // shared memory per team (the PRT kernel holds 9 gradient components instead of 6)
@@ -1416,23 +1465,8 @@ private:
         raise_smem_limit(kfn, tpc * total);
         // one CTA per group of tpc elements: measured faster on B200 than a persistent grid
         // (the hardware scheduler refills an SM as soon as any CTA ends, which hides the
-        // tail of uneven nr better than a fixed walk). AXG_PERSISTENT_GRID restores the
-        // persistent walk with next-element L2 prefetch.
+        // tail of uneven nr better than a fixed walk)
         b.grid = (b.n + tpc - 1) / tpc;
-        b.ahead = 0;
-#if AXG_PREFETCH_AHEAD > 0
-        if (!cfg_.plain && !b.prt) {
-            int per_sm = 0;
-            AXG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, team * tpc, tpc * total));
-            b.ahead = AXG_PREFETCH_AHEAD * std::max(per_sm, 1) * prop_.multiProcessorCount * tpc;
-        }
-#endif
-#ifdef AXG_PERSISTENT_GRID
-        int per_sm = 0;
-        AXG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, team * tpc, tpc * total));
-        if (!cfg_.plain && !b.prt)
-            b.grid = std::max(1, std::min(b.grid, std::max(1, per_sm) * prop_.multiProcessorCount));
-#endif
     }
 
     // The project's autotuner: for every solid bucket, time each feasible team size
@@ -1446,9 +1480,9 @@ private:
         for (auto &bp : sb_) {
             SolidBucket &b = *bp;
             float best = 1e30f;
-            int best_team = b.team;
-            for (int team : {32, 64, 128, 256}) {
-                b.team = team;
+            int best_team = b.kernel1d ? 0 : b.team;
+            for (int team : {0, 32, 64, 128, 256}) {
+                if (team == 0 && !b.kernel1d) continue;   // 1-D buckets: the default tiles as well
                 configure_bucket(b, team);
                 float ms = 0;
                 for (int rep = 0; rep < 3; rep++) {
@@ -1463,7 +1497,7 @@ private:
                 if (ms < best) { best = ms; best_team = team; }
             }
             configure_bucket(b, best_team);
-            tuned_.push_back({b.cls, best_team, best / 2});
+            tuned_.push_back({b.cls, b.team, best / 2});
         }
         cudaEventDestroy(t0);
         cudaEventDestroy(t1);
@@ -2132,7 +2166,13 @@ private:
         } else {
             SolidArgs<T, AT> af = a;
             af.fft_min_nr = b.fft ? AXG_FFT_MIN_NR : 0;
-            af.prefetch_ahead = b.ahead;
+            af.tab = b.tab.p;
+            af.tiles = b.tiles.p;
+            if (b.kernel1d) {
+                dim3 g = wave_grid(b.grid);
+                g.y = std::min(g.y, (unsigned)a.nwave);
+                b.kernel1d<<<g, b.team, b.team_bytes, ls()>>>(af, b.mt);
+            } else
             b.kernel<<<b.grid, b.team * b.tpc, b.tpc * b.team_bytes, ls()>>>(af, b.nr_max, b.qc, b.mt, b.tpc,
                                                                               b.team_bytes);
         }

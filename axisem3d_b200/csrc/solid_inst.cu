@@ -6,38 +6,58 @@ namespace axg {
 
 // NS: the register-resident SLS recursions are built for 3 and 5 SLS (3-D slices and
 // 1-D Fourier slots); other counts take the generic path
-template <class T, class AT, int RHEO, int ATT, bool IS3D, bool RTZ>
-static SolidKernel<T, AT> pick4(int nsls, bool fft) {
+template <class T, class AT, int RHEO, int ATT, bool RTZ>
+static SolidKernel<T, AT> pick3(int nsls, bool fft) {
 #ifndef AXG_GENERIC_SLS_ONLY
     if constexpr (ATT != ATT_NONE) {
-        if constexpr (IS3D) {
-            if (fft && nsls == 3) return solid_stiffness_kernel<T, AT, RHEO, ATT, IS3D, RTZ, 3, true>;
-            if (fft && nsls == 5) return solid_stiffness_kernel<T, AT, RHEO, ATT, IS3D, RTZ, 5, true>;
-        }
-        if (nsls == 3) return solid_stiffness_kernel<T, AT, RHEO, ATT, IS3D, RTZ, 3>;
-        if (nsls == 5) return solid_stiffness_kernel<T, AT, RHEO, ATT, IS3D, RTZ, 5>;
+        if (fft && nsls == 3) return solid_stiffness_kernel<T, AT, RHEO, ATT, RTZ, 3, true>;
+        if (fft && nsls == 5) return solid_stiffness_kernel<T, AT, RHEO, ATT, RTZ, 5, true>;
+        if (nsls == 3) return solid_stiffness_kernel<T, AT, RHEO, ATT, RTZ, 3>;
+        if (nsls == 5) return solid_stiffness_kernel<T, AT, RHEO, ATT, RTZ, 5>;
     }
 #endif
-    if constexpr (IS3D && ATT == ATT_NONE) {
-        if (fft) return solid_stiffness_kernel<T, AT, RHEO, ATT, IS3D, RTZ, 0, true>;
+    if constexpr (ATT == ATT_NONE) {
+        if (fft) return solid_stiffness_kernel<T, AT, RHEO, ATT, RTZ, 0, true>;
     }
-    return solid_stiffness_kernel<T, AT, RHEO, ATT, IS3D, RTZ, 0>;
+    return solid_stiffness_kernel<T, AT, RHEO, ATT, RTZ, 0>;
 }
-template <class T, class AT, int RHEO, int ATT, bool IS3D>
-static SolidKernel<T, AT> pick3(bool rtz, int nsls, bool fft) {
-    if constexpr (RHEO == RHEO_ISO) return pick4<T, AT, RHEO, ATT, IS3D, false>(nsls, fft);
-    else return rtz ? pick4<T, AT, RHEO, ATT, IS3D, true>(nsls, fft) : pick4<T, AT, RHEO, ATT, IS3D, false>(nsls, fft);
+template <class T, class AT, int RHEO, int ATT, bool RTZ>
+static Solid1DKernel<T, AT> pick3_1d(int nsls) {
+#ifndef AXG_GENERIC_SLS_ONLY
+    if constexpr (ATT != ATT_NONE) {
+        if (nsls == 3) return solid_1d_kernel<T, AT, RHEO, ATT, RTZ, 3>;
+        if (nsls == 5) return solid_1d_kernel<T, AT, RHEO, ATT, RTZ, 5>;
+    }
+#endif
+    return solid_1d_kernel<T, AT, RHEO, ATT, RTZ, 0>;
+}
+// isotropic stress is the same in both frames: no RTZ instantiation
+template <class T, class AT, int RHEO, int ATT>
+static SolidKernel<T, AT> pick2(bool rtz, int nsls, bool fft) {
+    if constexpr (RHEO != RHEO_ISO)
+        if (rtz) return pick3<T, AT, RHEO, ATT, true>(nsls, fft);
+    return pick3<T, AT, RHEO, ATT, false>(nsls, fft);
 }
 template <class T, class AT, int RHEO, int ATT>
-static SolidKernel<T, AT> pick2(bool is3d, bool rtz, int nsls, bool fft) {
-    return is3d ? pick3<T, AT, RHEO, ATT, true>(rtz, nsls, fft) : pick3<T, AT, RHEO, ATT, false>(rtz, nsls, fft);
+static Solid1DKernel<T, AT> pick2_1d(bool rtz, int nsls) {
+    if constexpr (RHEO != RHEO_ISO)
+        if (rtz) return pick3_1d<T, AT, RHEO, ATT, true>(nsls);
+    return pick3_1d<T, AT, RHEO, ATT, false>(nsls);
 }
 template <class T, class AT, int RHEO>
-SolidKernel<T, AT> pick_solid_of(int att, bool is3d, bool rtz, int nsls, bool fft) {
+SolidKernel<T, AT> pick_solid_of(int att, bool rtz, int nsls, bool fft) {
     switch (att) {
-        case ATT_NONE: return pick2<T, AT, RHEO, ATT_NONE>(is3d, rtz, nsls, fft);
-        case ATT_FULL: return pick2<T, AT, RHEO, ATT_FULL>(is3d, rtz, nsls, fft);
-        default: return pick2<T, AT, RHEO, ATT_CG4>(is3d, rtz, nsls, fft);
+        case ATT_NONE: return pick2<T, AT, RHEO, ATT_NONE>(rtz, nsls, fft);
+        case ATT_FULL: return pick2<T, AT, RHEO, ATT_FULL>(rtz, nsls, fft);
+        default: return pick2<T, AT, RHEO, ATT_CG4>(rtz, nsls, fft);
+    }
+}
+template <class T, class AT, int RHEO>
+Solid1DKernel<T, AT> pick_solid_1d_of(int att, bool rtz, int nsls) {
+    switch (att) {
+        case ATT_NONE: return pick2_1d<T, AT, RHEO, ATT_NONE>(rtz, nsls);
+        case ATT_FULL: return pick2_1d<T, AT, RHEO, ATT_FULL>(rtz, nsls);
+        default: return pick2_1d<T, AT, RHEO, ATT_CG4>(rtz, nsls);
     }
 }
 
@@ -55,8 +75,10 @@ PrtKernel<T, AT> pick_prt_of(int att, bool is3d, bool rtz) {
     }
 }
 
-template SolidKernel<AXG_INST_T, AXG_INST_AT> pick_solid_of<AXG_INST_T, AXG_INST_AT, AXG_INST_RHEO>(int, bool, bool,
-                                                                                                   int, bool);
+template SolidKernel<AXG_INST_T, AXG_INST_AT> pick_solid_of<AXG_INST_T, AXG_INST_AT, AXG_INST_RHEO>(int, bool, int,
+                                                                                                   bool);
+template Solid1DKernel<AXG_INST_T, AXG_INST_AT> pick_solid_1d_of<AXG_INST_T, AXG_INST_AT, AXG_INST_RHEO>(int, bool,
+                                                                                                        int);
 template PrtKernel<AXG_INST_T, AXG_INST_AT> pick_prt_of<AXG_INST_T, AXG_INST_AT, AXG_INST_RHEO>(int, bool, bool);
 
 }  // namespace axg

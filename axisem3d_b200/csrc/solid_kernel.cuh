@@ -1,4 +1,5 @@
-// solid_kernel.cuh -- fused stiffness of solid spectral elements (nPol = 4).
+// solid_kernel.cuh -- fused stiffness of solid spectral elements (nPol = 4) with properties per
+// azimuthal slice (3-D elements; those without are in solid1d_kernel.cuh).
 //
 // One team of threads evaluates one element at a time, entirely on chip:
 //   gather u from the points (zero-padded above each point's nu)
@@ -6,8 +7,7 @@
 //   GLL gradient + analytic d/dphi, axial L'Hopital rows
 //     GradientQuadrature::computeGrad6    (SOLVER/src/core/element/grad/GradientQuadrature.hpp:207-231)
 //   [RTZ] CoordTransformSpherical::transformSPZ_RTZ6 (crd/CoordTransformSpherical.hpp:186-216)
-//   1-D material: strainToStress_FR per Fourier mode
-//   3-D material: Fourier -> phi slices (direct DFT in shared memory, FFTW conventions,
+//   Fourier -> phi slices (direct DFT in shared memory, FFTW conventions,
 //     SOLVER/src/core/fft/SolverFFTW.hpp:101-172), strainToStress_CD per slice,
 //     slices -> Fourier
 //   Isotropic / TransverselyIsotropic / Anisotropic::strainToStress
@@ -43,14 +43,6 @@ constexpr int ATT_NONE = 0, ATT_FULL = 1, ATT_CG4 = 2;
 #ifndef AXG_SOLID_MIN_BLOCKS
 #define AXG_SOLID_MIN_BLOCKS 2
 #endif
-#ifndef AXG_PREFETCH_NEXT
-#define AXG_PREFETCH_NEXT 0
-#endif
-// 1 = the register-resident slice path sums slices k and nr - k together (a pass of its
-// own); 0 = one Fourier -> slice sum per (slice, point) inside the stress pass
-#ifndef AXG_SLICE_PAIRS
-#define AXG_SLICE_PAIRS 1
-#endif
 #ifndef AXG_KP
 #define AXG_KP 2
 #endif
@@ -61,29 +53,6 @@ constexpr int ATT_NONE = 0, ATT_FULL = 1, ATT_CG4 = 2;
 #endif
 #ifndef AXG_AB_ELASTIC
 #define AXG_AB_ELASTIC 4
-#endif
-// 1 = the stress pass of 3-D elements streams the SLS state of a (slice, point) in two
-// groups of three stress components (the recursion acts on each component alone), so that
-// 12 state words are live at a time instead of 24; 0 = the whole state loaded at once
-#ifndef AXG_SLS_SPLIT
-#define AXG_SLS_SPLIT 0
-#endif
-// > 0: each team prefetches into L2 the operands of the element AXG_PREFETCH_AHEAD waves of
-// resident CTAs ahead (the distance in SolidArgs::prefetch_ahead)
-#ifndef AXG_PREFETCH_AHEAD
-#define AXG_PREFETCH_AHEAD 0
-#endif
-// 1 = attenuating 3-D elements on the direct sums run the Fourier -> slice sums and the stress
-// pass as one pass: a thread per (slice pair, point) loads the operands of slice k, forms slices
-// k and nr - k, and applies stress and SLS recursion to both (one barrier less, no strain slices
-// through shared memory, the first slice's loads under the sums)
-#ifndef AXG_FUSED_SLICE
-#define AXG_FUSED_SLICE 0
-#endif
-// 1 = the stress pass's first (slice, point) of each thread has its SLS state loaded before the
-// Fourier -> slice pass (its latency hidden under that pass)
-#ifndef AXG_STATE_EARLY
-#define AXG_STATE_EARLY 0
 #endif
 // 1 = L2 prefetch of an element's slice operands (moduli, attenuation moduli, SLS state)
 // at the start of its slice phase
@@ -98,16 +67,6 @@ constexpr int ATT_NONE = 0, ATT_FULL = 1, ATT_CG4 = 2;
 #ifndef AXG_COLUMN_TILES
 #define AXG_COLUMN_TILES 1
 #endif
-// 1 = in FP32 arithmetic (the FP32 and mixed modes) the two direct-sum passes of a chunk of all
-// 25 points run on the tensor cores as small matrix products, (columns x modes) x (modes x
-// slice pairs) and (columns x slice pairs) x (slice pairs x modes), each operand split into a
-// TF32 head and tail and three products accumulated in FP32 (head x head + head x tail +
-// tail x head: the FP32 accuracy of the direct sums); the slice -> Fourier pass only outside
-// RTZ elements. Warp-level mma.sync tiles: parity holds, but measured slower than the column-
-// tiled FP32 sums on B200, so off
-#ifndef AXG_TC_DFT
-#define AXG_TC_DFT 0
-#endif
 // unrolling of the mode loop (Fourier -> slice) and of the slice loop (slice -> Fourier) of
 // the column-tiled passes
 #ifndef AXG_DFT_UNROLL
@@ -117,29 +76,6 @@ constexpr int KP = AXG_KP;   // slice pairs per thread in the paired Fourier -> 
 constexpr int KB = AXG_KB;   // slices per thread in the Fourier -> slice transform
 constexpr int AB = AXG_AB;   // modes per thread in the slice -> Fourier transform
 constexpr int DFT_UNROLL = AXG_DFT_UNROLL;
-
-// The SLS state is read once and written once per step: with AXG_STREAM_STATE its loads and
-// stores carry the streaming cache hint (evict first), so that it does not push the moduli and
-// the point fields out of L2.
-#ifndef AXG_STREAM_STATE
-#define AXG_STREAM_STATE 0
-#endif
-template <class AT>
-__device__ __forceinline__ AT state_ld(const AT *p) {
-#if AXG_STREAM_STATE
-    return __ldcs(p);
-#else
-    return *p;
-#endif
-}
-template <class AT>
-__device__ __forceinline__ void state_st(AT *p, AT v) {
-#if AXG_STREAM_STATE
-    __stcs(p, v);
-#else
-    *p = v;
-#endif
-}
 
 template <class T, class AT>
 struct SolidArgs {
@@ -168,14 +104,14 @@ struct SolidArgs {
     size_t fstride;            // complex values between wavefields in displ / stiff
     size_t sstride;            // AT values between wavefields in the state pool
     int fft_min_nr;            // 3-D elements with nr >= this (and 13-smooth nr) take the FFT; 0 = never
-    int prefetch_ahead;        // > 0: each team prefetches into L2 the operands of the element this
-                               // many places ahead (about one wave of resident CTAs); 0 = off
+    const int2 *tab;           // [n][25] first mode and number of modes of the element's points
+    const int4 *tiles;         // 1-D elements: (element, first mode, modes, nu | axial << 30) per block
 };
 
 // shared memory layout of one team
 struct TeamLayout {
     int nr_max, nu_max, qc;
-    size_t geom, trig, ipt, tw, tws, regA, regB, total;
+    size_t geom, trig, ipt, tw, regA, regB, total;
 };
 
 template <class T>
@@ -191,8 +127,6 @@ __host__ __device__ inline TeamLayout team_layout(int nr_max, int qc, int mt) {
     L.trig = o; o = al(o + 4 * 25 * sizeof(T));
     L.ipt = o;  o = al(o + 3 * 25 * sizeof(int));
     L.tw = o;   o = al(o + 2 * (size_t)nr_max * sizeof(T));
-    // the twiddles split for the tensor-core sums: (cos head, cos tail, sin head, sin tail)
-    L.tws = o;  o = al(o + (AXG_TC_DFT && sizeof(T) == 4 ? 4 * (size_t)nr_max * sizeof(T) : 0));
     L.regA = o; o = al(o + 6 * (size_t)L.nu_max * 25 * 2 * sizeof(T));
     size_t b1 = 3 * (size_t)mt * 25 * 2 * sizeof(T);
     size_t b2 = (size_t)nr_max * 6 * qc * sizeof(T);
@@ -245,171 +179,6 @@ __device__ __forceinline__ void st6r(T *p, const T (&v)[6]) {
     cx_t<T> *q = reinterpret_cast<cx_t<T> *>(p);
 #pragma unroll
     for (int i = 0; i < 3; i++) q[i] = mk<T>(v[2 * i], v[2 * i + 1]);
-}
-
-// ------------------------------------------------- tensor-core direct sums ---
-// TF32 head of x (round to nearest, ties away: exact in TF32, whatever the tensor core does with
-// the low 13 bits of an operand) and the tail x - head (exact in FP32; its own rounding to TF32
-// costs at most 2^-22 |x|)
-__device__ __forceinline__ uint32_t tf32_head(float x) {
-    uint32_t r;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-    return r;
-}
-__device__ __forceinline__ void tf32_split(float x, uint32_t &h, uint32_t &t) {
-    h = tf32_head(x);
-    t = tf32_head(x - __uint_as_float(h));
-}
-// d += a b for one m16n8k8 tile: a (16 x 8, row-major fragment: a0 (g, c), a1 (g + 8, c),
-// a2 (g, c + 4), a3 (g + 8, c + 4)), b (8 x 8: b0 (c, g), b1 (c + 4, g)), d (16 x 8: d0 (g, 2c),
-// d1 (g, 2c + 1), d2 (g + 8, 2c), d3 (g + 8, 2c + 1)); g = lane / 4, c = lane % 4
-__device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-        "{%0,%1,%2,%3};\n"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-// (ah + at) (bh + bt) without the tail x tail product, into three accumulators (head x head,
-// and the two cross terms) so that the three products do not wait on one another
-__device__ __forceinline__ void mma_tf32x3(float (&d)[3][4], const uint32_t (&ah)[4], const uint32_t (&at)[4],
-                                           uint32_t bh0, uint32_t bh1, uint32_t bt0, uint32_t bt1) {
-    mma_tf32(d[0], ah, bh0, bh1);
-    mma_tf32(d[1], at, bh0, bh1);
-    mma_tf32(d[2], ah, bt0, bt1);
-}
-// x mod n for 0 <= x < 2^22 with rn = 1 / n (a float quotient off by at most one, corrected)
-__device__ __forceinline__ int mod_n(int x, int n, float rn) {
-    int r = x - (int)((float)x * rn) * n;
-    r += r < 0 ? n : 0;
-    return r >= n ? r - n : r;
-}
-
-// Fourier -> slices of a chunk holding all 25 points, on the tensor cores. Rows n = d * 25 + q of
-// the (component, point) block (10 tiles of 16), columns k = slice pairs 0 .. nr/2 (tiles of 8),
-// modes a = 1 .. nu - 1 in steps of 8: A[n][k] = sum_a Re c_a[n] cos(a k 2pi/nr) and
-// B[n][k] = sum_a Im c_a[n] sin(a k 2pi/nr), then x_k = c0 + 2 (A - B), x_{nr-k} = c0 + 2 (A + B)
-// (the paired direct sums, each product in three TF32 parts)
-template <class T>
-__device__ __forceinline__ void tc_fourier_to_slices(const cx_t<T> *rA, T *rBr, const float4 *tws, int nr,
-                                                     int lane, int TEAM) {
-    if constexpr (sizeof(T) == 4) {
-        const int nu = nr / 2 + 1;
-        const int wi = lane >> 5, nw = TEAM >> 5, g = (lane & 31) >> 2, c = lane & 3;
-        const int NT = (nu + 7) >> 3, KS = (nu - 1 + 7) >> 3;
-        const float rnr = 1.f / (float)nr;
-        for (int t = wi; t < 10 * NT; t += nw) {
-            const int mt = t % 10, nt = t / 10;
-            const int n0 = mt * 16 + g, n1 = n0 + 8, kp = nt * 8 + g;
-            float dA[3][4] = {}, dB[3][4] = {};
-            // twiddle indices (a k) mod nr of this thread's two B rows, modes 1 + c and 5 + c
-            int j0 = mod_n((1 + c) * kp, nr, rnr), j1 = mod_n((5 + c) * kp, nr, rnr);
-            const int s8 = mod_n(8 * kp, nr, rnr);
-            for (int ks = 0; ks < KS; ks++) {
-                const int a0 = 1 + 8 * ks + c, a1 = a0 + 4;
-                const float2 z = make_float2(0.f, 0.f);
-                float2 v[4];
-                v[0] = (a0 < nu && n0 < 150) ? rA[a0 * 150 + n0] : z;
-                v[1] = (a0 < nu && n1 < 150) ? rA[a0 * 150 + n1] : z;
-                v[2] = (a1 < nu && n0 < 150) ? rA[a1 * 150 + n0] : z;
-                v[3] = (a1 < nu && n1 < 150) ? rA[a1 * 150 + n1] : z;
-                uint32_t rh[4], rt[4], ih[4], it[4];
-#pragma unroll
-                for (int r = 0; r < 4; r++) {
-                    tf32_split(v[r].x, rh[r], rt[r]);
-                    tf32_split(v[r].y, ih[r], it[r]);
-                }
-                const float4 w0 = tws[j0], w1 = tws[j1];
-                mma_tf32x3(dA, rh, rt, __float_as_uint(w0.x), __float_as_uint(w1.x), __float_as_uint(w0.y),
-                           __float_as_uint(w1.y));
-                mma_tf32x3(dB, ih, it, __float_as_uint(w0.z), __float_as_uint(w1.z), __float_as_uint(w0.w),
-                           __float_as_uint(w1.w));
-                j0 += s8;
-                j0 = j0 >= nr ? j0 - nr : j0;
-                j1 += s8;
-                j1 = j1 >= nr ? j1 - nr : j1;
-            }
-#pragma unroll
-            for (int r = 0; r < 4; r++) {
-                const int n = r < 2 ? n0 : n1, k = nt * 8 + 2 * c + (r & 1);
-                if (n < 150 && k < nu) {
-                    const float c0 = rA[n].x;
-                    const float A = dA[0][r] + (dA[1][r] + dA[2][r]), B = dB[0][r] + (dB[1][r] + dB[2][r]);
-                    rBr[k * 150 + n] = c0 + 2.f * (A - B);
-                    if (k != 0 && 2 * k != nr) rBr[(nr - k) * 150 + n] = c0 + 2.f * (A + B);
-                }
-            }
-        }
-    }
-}
-
-// slices -> Fourier of a chunk holding all 25 points, on the tensor cores: rows n of the block,
-// columns a = 0 .. nu - 1 (tiles of 8), slice pairs k = 0 .. nr/2 in steps of 8:
-// Re S_a[n] = sum_k xs_k[n] cos(a k 2pi/nr) / nr, Im S_a[n] = -sum_k xd_k[n] sin(a k 2pi/nr) / nr
-// with xs_k = x_k + x_{nr-k}, xd_k = x_k - x_{nr-k} (x_k alone at k = 0 and nr/2), the Nyquist
-// mode halved and the imaginary parts of modes 0 and nr/2 dropped
-template <class T>
-__device__ __forceinline__ void tc_slices_to_fourier(cx_t<T> *rA, const T *rBr, const float4 *tws, int nr,
-                                                     T inv_nr, int lane, int TEAM) {
-    if constexpr (sizeof(T) == 4) {
-        const int nu = nr / 2 + 1;
-        const int wi = lane >> 5, nw = TEAM >> 5, g = (lane & 31) >> 2, c = lane & 3;
-        const int NT = (nu + 7) >> 3, KS = (nu + 7) >> 3;
-        const float rnr = 1.f / (float)nr;
-        auto sd = [&](int k, int n, float &xs, float &xd) {
-            xs = 0.f;
-            xd = 0.f;
-            if (k < nu && n < 150) {
-                const float x1 = rBr[k * 150 + n];
-                xs = x1;
-                if (k != 0 && 2 * k != nr) {
-                    const float x2 = rBr[(nr - k) * 150 + n];
-                    xs = x1 + x2;
-                    xd = x1 - x2;
-                }
-            }
-        };
-        for (int t = wi; t < 10 * NT; t += nw) {
-            const int mt = t % 10, nt = t / 10;
-            const int n0 = mt * 16 + g, n1 = n0 + 8, am = nt * 8 + g;
-            float dC[3][4] = {}, dS[3][4] = {};
-            // twiddle indices (k a) mod nr of this thread's two B rows, slices c and c + 4
-            int j0 = mod_n(c * am, nr, rnr), j1 = mod_n((c + 4) * am, nr, rnr);
-            const int s8 = mod_n(8 * am, nr, rnr);
-            for (int ks = 0; ks < KS; ks++) {
-                const int k0 = 8 * ks + c, k1 = k0 + 4;
-                float xs[4], xd[4];
-                sd(k0, n0, xs[0], xd[0]);
-                sd(k0, n1, xs[1], xd[1]);
-                sd(k1, n0, xs[2], xd[2]);
-                sd(k1, n1, xs[3], xd[3]);
-                uint32_t sh[4], st[4], dh[4], dt[4];
-#pragma unroll
-                for (int r = 0; r < 4; r++) {
-                    tf32_split(xs[r], sh[r], st[r]);
-                    tf32_split(xd[r], dh[r], dt[r]);
-                }
-                const float4 w0 = tws[j0], w1 = tws[j1];
-                mma_tf32x3(dC, sh, st, __float_as_uint(w0.x), __float_as_uint(w1.x), __float_as_uint(w0.y),
-                           __float_as_uint(w1.y));
-                mma_tf32x3(dS, dh, dt, __float_as_uint(w0.z), __float_as_uint(w1.z), __float_as_uint(w0.w),
-                           __float_as_uint(w1.w));
-                j0 += s8;
-                j0 = j0 >= nr ? j0 - nr : j0;
-                j1 += s8;
-                j1 = j1 >= nr ? j1 - nr : j1;
-            }
-#pragma unroll
-            for (int r = 0; r < 4; r++) {
-                const int n = r < 2 ? n0 : n1, al = nt * 8 + 2 * c + (r & 1);
-                if (n < 150 && al < nu) {
-                    const bool nyq = (nr & 1) == 0 && al == nr / 2;
-                    const float re = (dC[0][r] + (dC[1][r] + dC[2][r])) * (nyq ? 0.5f * inv_nr : inv_nr);
-                    const float im = (al == 0 || nyq) ? 0.f : -(dS[0][r] + (dS[1][r] + dS[2][r])) * inv_nr;
-                    rA[al * 150 + n] = make_float2(re, im);
-                }
-            }
-        }
-    }
 }
 
 // ------------------------------------------------------------ rheology ---
@@ -582,21 +351,6 @@ __device__ __forceinline__ void prefetch_l2(const void *p, size_t bytes, int lan
     for (; a < a1; a += (uintptr_t)team * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(a));
 }
 
-// bytes of the per-element streams (geometry, moduli, attenuation moduli, state)
-template <class T, class AT, int RHEO, int ATT, bool IS3D>
-__device__ __forceinline__ void prefetch_element(const SolidArgs<T, AT> &a, int e, int lane, int team) {
-    const int nr = a.nr[e], nu = nr / 2 + 1, ns = IS3D ? nr : 1;
-    constexpr int nmod = RHEO == RHEO_ISO ? 2 : RHEO == RHEO_TISO ? 5 : 21;
-    prefetch_l2(a.geom + (size_t)e * 250, 250 * sizeof(T), lane, team);
-    prefetch_l2(a.mod + a.mod_off[e], (size_t)nmod * ns * 25 * sizeof(T), lane, team);
-    if constexpr (ATT != ATT_NONE) {
-        constexpr int npa = ATT == ATT_CG4 ? 4 : 25;
-        prefetch_l2(a.attmod + a.att_off[e], (size_t)2 * ns * npa * sizeof(T), lane, team);
-        const size_t slots = IS3D ? (size_t)nr * npa : (size_t)nu * npa * 2;
-        prefetch_l2(a.state + a.state_off[e], (size_t)(a.nsls + 1) * 6 * slots * sizeof(AT), lane, team);
-    }
-}
-
 // SLS recursion on one real slice point with the state already in registers
 // (same steps and order as attenuate<>; NS = number of SLS, a compile-time size)
 template <int NS, class T, class AT>
@@ -627,121 +381,6 @@ __device__ __forceinline__ void attenuate_regs(const AT *alpha, const AT *beta, 
         for (int d = 0; d < 6; d++) mem[l][d] += gamma[l] * ds[d];
 #pragma unroll
     for (int d = 0; d < 6; d++) s[d] = (T)sv[d];
-}
-
-// SLS recursion on one real slice point with the state streamed from memory in two groups of
-// three stress components, (0, 1, 2) then (3, 4, 5): each group loads its 3 + 3 NS words at once,
-// updates them with the steps and order of attenuate_regs (per component the same operations,
-// so the same results) and stores them back. State word j of the slot is at j * nslot + slot.
-template <int NS, class T, class AT>
-__device__ __forceinline__ void attenuate_slice_split(const AT *alpha, const AT *beta, const AT *gamma, AT *st,
-                                                      size_t nslot, size_t slot, const T e[6], T s[6], T dl,
-                                                      T dm) {
-    const AT lam = (AT)dl, mu = (AT)dm, mu2 = mu + mu;
-#pragma unroll
-    for (int g = 0; g < 2; g++) {
-        const int d0 = 3 * g;
-        AT ds[3], mem[NS][3];
-#pragma unroll
-        for (int c = 0; c < 3; c++) ds[c] = state_ld(st + (d0 + c) * nslot + slot);
-#pragma unroll
-        for (int l = 0; l < NS; l++)
-#pragma unroll
-            for (int c = 0; c < 3; c++) mem[l][c] = state_ld(st + (6 + l * 6 + d0 + c) * nslot + slot);
-        AT dn[3];
-        if (g == 0) {
-            const AT e0 = (AT)e[0], e1 = (AT)e[1], e2 = (AT)e[2];
-            const AT sii = (e0 + e1 + e2) * lam;
-            dn[0] = sii + e0 * mu2;
-            dn[1] = sii + e1 * mu2;
-            dn[2] = sii + e2 * mu2;
-        } else {
-#pragma unroll
-            for (int c = 0; c < 3; c++) dn[c] = (AT)e[3 + c] * mu;
-        }
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-            AT sv = (AT)s[d0 + c];
-#pragma unroll
-            for (int l = 0; l < NS; l++) {
-                sv -= mem[l][c];
-                mem[l][c] = alpha[l] * mem[l][c] + beta[l] * ds[c];
-            }
-#pragma unroll
-            for (int l = 0; l < NS; l++) mem[l][c] += gamma[l] * dn[c];
-            s[d0 + c] = (T)sv;
-            state_st(st + (d0 + c) * nslot + slot, dn[c]);
-        }
-#pragma unroll
-        for (int l = 0; l < NS; l++)
-#pragma unroll
-            for (int c = 0; c < 3; c++) state_st(st + (6 + l * 6 + d0 + c) * nslot + slot, mem[l][c]);
-    }
-}
-
-// SLS recursion on one complex Fourier-space slot of a 1-D element, state in registers. The
-// recursion is linear and acts on each stress component separately, on the real and the
-// imaginary parts alike, so the slot runs in four passes: (real, imaginary) x (components
-// 0-2, which share the trace of the strain, and 3-5). Each pass loads its 3 + 3 NS state
-// words at once (independent loads whose latencies overlap), updates them in registers with
-// the steps and order of attenuate_regs, and stores them back. Same layout and results as
-// attenuate<T, AT, true>: part w of state word j of the slot is at (j * nslot + slot) * 2 + w.
-template <int NS, class T, class AT>
-__device__ __forceinline__ void attenuate_cplx_regs(const SolidArgs<T, AT> &a, AT *state, size_t nslot,
-                                                    size_t slot, const cx_t<T> e[6], cx_t<T> s[6], T dl,
-                                                    T dm) {
-    const AT lam = (AT)dl, mu = (AT)dm, mu2 = mu + mu;
-#pragma unroll 1
-    for (int pass = 0; pass < 4; pass++) {
-        const int w = pass & 1, d0 = (pass >> 1) * 3;
-        AT *base = state + w;
-        AT ds[3], mem[NS][3];
-#pragma unroll
-        for (int c = 0; c < 3; c++) ds[c] = base[((d0 + c) * nslot + slot) * 2];
-#pragma unroll
-        for (int l = 0; l < NS; l++)
-#pragma unroll
-            for (int c = 0; c < 3; c++) mem[l][c] = base[((6 + l * 6 + d0 + c) * nslot + slot) * 2];
-        // new dstress of these components (Isotropic::strainToStress with dlambda, dmu)
-        AT dn[3];
-        if (d0 == 0) {
-            const AT e0 = (AT)(w ? e[0].y : e[0].x), e1 = (AT)(w ? e[1].y : e[1].x),
-                     e2 = (AT)(w ? e[2].y : e[2].x);
-            const AT sii = (e0 + e1 + e2) * lam;
-            dn[0] = sii + e0 * mu2;
-            dn[1] = sii + e1 * mu2;
-            dn[2] = sii + e2 * mu2;
-        } else {
-#pragma unroll
-            for (int c = 0; c < 3; c++) dn[c] = (AT)(w ? e[3 + c].y : e[3 + c].x) * mu;
-        }
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-            AT sv = (AT)(w ? s[d0 + c].y : s[d0 + c].x);
-#pragma unroll
-            for (int l = 0; l < NS; l++) {
-                sv -= mem[l][c];
-                mem[l][c] = a.alpha[l] * mem[l][c] + a.beta[l] * ds[c];
-            }
-#pragma unroll
-            for (int l = 0; l < NS; l++) mem[l][c] += a.gamma[l] * dn[c];
-            if (w) s[d0 + c].y = (T)sv;
-            else s[d0 + c].x = (T)sv;
-            base[((d0 + c) * nslot + slot) * 2] = dn[c];
-        }
-#pragma unroll
-        for (int l = 0; l < NS; l++)
-#pragma unroll
-            for (int c = 0; c < 3; c++) base[((6 + l * 6 + d0 + c) * nslot + slot) * 2] = mem[l][c];
-    }
-}
-
-// 1-D elements: the register-resident recursion for 3 and 5 SLS, the generic one otherwise
-template <int NS, class T, class AT>
-__device__ __forceinline__ void attenuate_1d(const SolidArgs<T, AT> &a, AT *state, size_t nslot, size_t slot,
-                                             const cx_t<T> e[6], cx_t<T> s[6], T dl, T dm) {
-    if constexpr (NS > 0) attenuate_cplx_regs<NS, T, AT>(a, state, nslot, slot, e, s, dl, dm);
-    else attenuate<T, AT, true>(a, state, nslot, slot, e, s, dl, dm);
 }
 
 __device__ __forceinline__ int cg4_slot(int q) {
@@ -914,12 +553,11 @@ __device__ __forceinline__ FftView<T> fft_run(FftView<T> b0, FftView<T> b1, int 
 }
 
 // ----------------------------------------------------------------- kernel ---
-// NS: compile-time number of SLS for the register-resident recursions (the slice path of 3-D
-// elements, the Fourier-space path of 1-D elements); 0 = the generic path with the count
-// read at run time
-// FFT: the instantiation that holds the slice FFTs (3-D buckets with large nr); the others
+// NS: compile-time number of SLS for the register-resident recursion; 0 = the generic path with
+// the count read at run time
+// FFT: the instantiation that holds the slice FFTs (buckets with large nr); the others
 // keep only the direct sums, so the FFT code costs them no registers
-template <class T, class AT, int RHEO, int ATT, bool IS3D, bool RTZ, int NS, bool FFT = false>
+template <class T, class AT, int RHEO, int ATT, bool RTZ, int NS, bool FFT = false>
 __global__ void __launch_bounds__(256, AXG_SOLID_MIN_BLOCKS)
 solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_max, const int mt_max,
                        const int teams_per_cta, const size_t team_bytes) {
@@ -948,7 +586,6 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
     int *sOff = sPt + 25;
     int *sNu = sPt + 50;
     T *sTw = reinterpret_cast<T *>(base + L.tw);
-    float4 *sTws = reinterpret_cast<float4 *>(base + L.tws);
     C *rA = reinterpret_cast<C *>(base + L.regA);
     C *rBc = reinterpret_cast<C *>(base + L.regB);
     T *rBr = reinterpret_cast<T *>(base + L.regB);
@@ -960,20 +597,11 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
             *dzdeta_if = sGeo + 200, *invs_if = sGeo + 225;
 
     const int stride = gridDim.x * teams_per_cta;
-    if (AXG_PREFETCH_NEXT && blockIdx.x * teams_per_cta + team < a.n_elem)
-        prefetch_element<T, AT, RHEO, ATT, IS3D>(a, blockIdx.x * teams_per_cta + team, lane, TEAM);
     for (int e = blockIdx.x * teams_per_cta + team; e < a.n_elem; e += stride) {
         const int nr = a.nr[e];
         const int nu = nr / 2 + 1;
         const bool axial = a.axial[e] != 0;
         const T *Gxi = axial ? sGlj : sGll;
-        // the next element of this team streams into L2 while this one computes
-        if (AXG_PREFETCH_NEXT && e + stride < a.n_elem)
-            prefetch_element<T, AT, RHEO, ATT, IS3D>(a, e + stride, lane, TEAM);
-        // the element about one wave of resident CTAs ahead streams into L2 while this one computes
-        if (AXG_PREFETCH_AHEAD > 0 && a.prefetch_ahead > 0 && e + a.prefetch_ahead < a.n_elem)
-            prefetch_element<T, AT, RHEO, ATT, IS3D>(a, e + a.prefetch_ahead, lane, TEAM);
-
         // ---------------- element header -> shared memory ----------------
         for (int i = lane; i < 250; i += TEAM) sGeo[i] = a.geom[(size_t)e * 250 + i];
         if constexpr (RTZ)
@@ -984,19 +612,10 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
             sOff[i] = a.pt_off[p];
             sNu[i] = a.pt_nu[p];
         }
-        if constexpr (IS3D) {
+        {
             const T *tw = a.tw + a.tw_off[nr];
             // interleaved (cos, sin) pairs: one 2-word shared load per twiddle
             for (int i = lane; i < 2 * nr; i += TEAM) sTw[i] = (i & 1) ? tw[nr + (i >> 1)] : tw[i >> 1];
-            if constexpr (AXG_TC_DFT && sizeof(T) == 4) {
-                for (int i = lane; i < nr; i += TEAM) {
-                    uint32_t ch, ct, sh, st;
-                    tf32_split((float)tw[i], ch, ct);
-                    tf32_split((float)tw[nr + i], sh, st);
-                    sTws[i] = make_float4(__uint_as_float(ch), __uint_as_float(ct), __uint_as_float(sh),
-                                          __uint_as_float(st));
-                }
-            }
         }
         team_sync(team, TEAM);
 
@@ -1005,16 +624,8 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
         const C *displw = a.displ + (size_t)w * a.fstride;
         C *stiffw = a.stiff + (size_t)w * a.fstride;
         AT *statew = a.state + (size_t)w * a.sstride;
-#if AXG_PREFETCH_SLICES
-        if constexpr (!IS3D && ATT != ATT_NONE && NS > 0) {
-            // the SLS state of this 1-D element starts moving into L2 now, so that the stress
-            // pass after the gather and the gradient finds it there
-            constexpr int NPA_ = ATT == ATT_CG4 ? 4 : 25;
-            prefetch_l2(statew + a.state_off[e], (size_t)(6 + 6 * NS) * nu * NPA_ * 2 * sizeof(AT), lane, TEAM);
-        }
-#endif
         const int64_t moff = a.mod_off[e];
-        const int nslice = IS3D ? nr : 1;
+        const int nslice = nr;
         for (int t0 = 0; t0 < nu; t0 += mt_max) {
         const int mt = min(mt_max, nu - t0);
         // ---------------- gather displacement: U[a - t0][c][q] in region B ----------------
@@ -1096,80 +707,14 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
             if constexpr (RTZ) {
                 spz_to_rtz6(eps, sTrig[q], sTrig[25 + q], sTrig[50 + q], sTrig[75 + q]);
             }
-            if constexpr (!IS3D && !(ATT != ATT_NONE && NS > 0)) {
-                // strainToStress_FR with 1-D moduli
-                C sig[6];
-                elastic_at<RHEO>(a.mod + moff, 1, 0, q, eps, sig);
-                if constexpr (ATT == ATT_FULL) {
-                    const int64_t ao = a.att_off[e];
-                    AT *st = statew + a.state_off[e];
-                    attenuate_1d<NS, T, AT>(a, st, (size_t)nu * 25, (size_t)al * 25 + q, eps, sig,
-                                           a.attmod[ao + q], a.attmod[ao + 25 + q]);
-                } else if constexpr (ATT == ATT_CG4) {
-                    const int k4 = cg4_slot(q);
-                    if (k4 >= 0) {
-                        const int64_t ao = a.att_off[e];
-                        AT *st = statew + a.state_off[e];
-                        attenuate_1d<NS, T, AT>(a, st, (size_t)nu * 4, (size_t)al * 4 + k4, eps, sig,
-                                               a.attmod[ao + k4], a.attmod[ao + 4 + k4]);
-                    }
-                }
-                if constexpr (RTZ) {
-                    rtz_to_spz6(sig, sTrig[q], sTrig[25 + q], sTrig[50 + q], sTrig[75 + q]);
-                }
 #pragma unroll
-                for (int d = 0; d < 6; d++) rA[(al * 6 + d) * 25 + q] = sig[d];
-            } else {
-#pragma unroll
-                for (int d = 0; d < 6; d++) rA[(al * 6 + d) * 25 + q] = eps[d];
-            }
+            for (int d = 0; d < 6; d++) rA[(al * 6 + d) * 25 + q] = eps[d];
         }
         team_sync(team, TEAM);
         }   // mode tiles of the gather + gradient
 
-        // ---------------- 1-D attenuation: stress pass, SLS state in registers ----------------
-        // strainToStress_FR on the strain left in region A, then the SLS recursion of each
-        // attenuating slot with its whole state loaded at once; with CG4 the recursion runs on
-        // threads mapped to the 4 CG4 points of each mode only
-        if constexpr (!IS3D && ATT != ATT_NONE && NS > 0) {
-            const int64_t ao = a.att_off[e];
-            AT *st = statew + a.state_off[e];
-            auto stress_slot = [&](int al, int q, bool att, size_t nslot, size_t slot, T dl, T dm) {
-                C ev[6], sig[6];
-#pragma unroll
-                for (int d = 0; d < 6; d++) ev[d] = rA[(al * 6 + d) * 25 + q];
-                elastic_at<RHEO>(a.mod + moff, 1, 0, q, ev, sig);
-                if (att) attenuate_cplx_regs<NS, T, AT>(a, st, nslot, slot, ev, sig, dl, dm);
-                if constexpr (RTZ) {
-                    rtz_to_spz6(sig, sTrig[q], sTrig[25 + q], sTrig[50 + q], sTrig[75 + q]);
-                }
-#pragma unroll
-                for (int d = 0; d < 6; d++) rA[(al * 6 + d) * 25 + q] = sig[d];
-            };
-            if constexpr (ATT == ATT_FULL) {
-                for (int i = lane; i < nu * 25; i += TEAM) {
-                    const int al = i / 25, q = i - al * 25;
-                    stress_slot(al, q, true, (size_t)nu * 25, (size_t)i, a.attmod[ao + q], a.attmod[ao + 25 + q]);
-                }
-            } else {
-                // CG4 points (1,1) (1,3) (3,1) (3,3) = 6, 8, 16, 18 of each mode
-                for (int i = lane; i < nu * 4; i += TEAM) {
-                    const int al = i >> 2, k4 = i & 3;
-                    const int q = 6 + 2 * (k4 & 1) + 10 * (k4 >> 1);
-                    stress_slot(al, q, true, (size_t)nu * 4, (size_t)i, a.attmod[ao + k4], a.attmod[ao + 4 + k4]);
-                }
-                // the other 21 points of each mode: elastic only
-                for (int i = lane; i < nu * 21; i += TEAM) {
-                    const int al = i / 21, j = i - al * 21;
-                    const int q = j + (j >= 6) + (j >= 7) + (j >= 14) + (j >= 15);
-                    stress_slot(al, q, false, 0, 0, (T)0, (T)0);
-                }
-            }
-            team_sync(team, TEAM);
-        }
-
         // ---------------- 3-D material: slices ----------------
-        if constexpr (IS3D) {
+        {
             using T2 = cx_t<T>;
             const T2 *tw2 = reinterpret_cast<const T2 *>(sTw);
             const T inv_nr = (T)1 / (T)nr;
@@ -1211,30 +756,6 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
                 constexpr int NPA = ATT == ATT_CG4 ? 4 : 25;
                 const T *modp = a.mod + moff;
                 const size_t nsl = (size_t)nslice * 25;
-#if AXG_STATE_EARLY
-                // the SLS state of this thread's first (slice, point) of the stress pass is
-                // loaded now, so that its latency runs under the Fourier -> slice pass
-                AT ds0[6], mem0[NSR][6];
-                bool pre = false;
-                if constexpr (ATT != ATT_NONE && NS > 0) {
-                    if (lane < nr * qcnt) {
-                        const int k = lane / qcnt, q = q0 + lane - k * qcnt;
-                        const int k4 = ATT == ATT_CG4 ? cg4_slot(q) : q;
-                        if (k4 >= 0) {
-                            const size_t nslot = (size_t)nr * NPA, slot = (size_t)k * NPA + k4;
-                            const AT *st = statew + a.state_off[e];
-#pragma unroll
-                            for (int d = 0; d < 6; d++) ds0[d] = state_ld(st + d * nslot + slot);
-#pragma unroll
-                            for (int l = 0; l < NSR; l++)
-#pragma unroll
-                                for (int d = 0; d < 6; d++) mem0[l][d] = state_ld(st + (6 + l * 6 + d) * nslot + slot);
-                            pre = true;
-                        }
-                    }
-                }
-#endif
-                bool fused_done = false;
                 if (FFT && use_fft) {
                     // Hermitian spectra of the component pairs, Z = Y_2p + i Y_2p+1 over all nr
                     // orders: Y_0 = Re c_0, Y_a = c_a, Y_nr-a = conj c_a, Y_nr/2 = 2 Re c_nr/2
@@ -1257,95 +778,6 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
                     // from here on the chunk's columns of region A are free until the unpacking
                     vs = fft_run<T>(vB, vA, nr, qcnt, plan, +1, tw2, team, lane, TEAM);
                 } else {
-#if AXG_FUSED_SLICE
-                if constexpr (ATT != ATT_NONE && NS > 0) {
-                    fused_done = true;
-                    const int npair = nr / 2 + 1;
-                    const size_t nslot = (size_t)nr * NPA;
-                    AT *st = statew + a.state_off[e];
-                    const T *am = a.attmod + a.att_off[e];
-                    // the operands of (slice k, point q): moduli, attenuation moduli, SLS state
-                    auto load_ops = [&](int k, int q, int k4, T (&md)[NM], T &dl, T &dmu, AT (&ds)[6],
-                                        AT (&mem)[NSR][6]) {
-#pragma unroll
-                        for (int mm = 0; mm < NM; mm++) md[mm] = __ldg(modp + mm * nsl + (size_t)k * 25 + q);
-                        if (k4 >= 0) {
-                            const size_t slot = (size_t)k * NPA + k4;
-                            dl = __ldg(am + slot);
-                            dmu = __ldg(am + nslot + slot);
-#pragma unroll
-                            for (int d = 0; d < 6; d++) ds[d] = state_ld(st + d * nslot + slot);
-#pragma unroll
-                            for (int l = 0; l < NSR; l++)
-#pragma unroll
-                                for (int d = 0; d < 6; d++) mem[l][d] = state_ld(st + (6 + l * 6 + d) * nslot + slot);
-                        }
-                    };
-                    // stress and SLS recursion of one slice; the stress to region B
-                    auto stress_slice = [&](int k, int qq, int k4, const T (&x)[6], const T (&md)[NM], T dl, T dmu,
-                                            AT (&ds)[6], AT (&mem)[NSR][6]) {
-                        re1<T> ev[6], sg[6];
-#pragma unroll
-                        for (int d = 0; d < 6; d++) ev[d].x = x[d];
-                        if constexpr (RHEO == RHEO_ISO) stress_iso(ev, sg, md[0], md[1]);
-                        else if constexpr (RHEO == RHEO_TISO) stress_tiso(ev, sg, md[0], md[1], md[2], md[3], md[4]);
-                        else stress_aniso(ev, sg, md);
-                        if (k4 >= 0) {
-                            const size_t slot = (size_t)k * NPA + k4;
-                            T e6[6], s6[6];
-#pragma unroll
-                            for (int d = 0; d < 6; d++) { e6[d] = ev[d].x; s6[d] = sg[d].x; }
-                            attenuate_regs<NSR, T, AT>(a.alpha, a.beta, a.gamma, ds, mem, e6, s6, dl, dmu);
-#pragma unroll
-                            for (int d = 0; d < 6; d++) sg[d].x = s6[d];
-#pragma unroll
-                            for (int d = 0; d < 6; d++) state_st(st + d * nslot + slot, ds[d]);
-#pragma unroll
-                            for (int l = 0; l < NSR; l++)
-#pragma unroll
-                                for (int d = 0; d < 6; d++) state_st(st + (6 + l * 6 + d) * nslot + slot, mem[l][d]);
-                        }
-#pragma unroll
-                        for (int d = 0; d < 6; d++) rBr[((size_t)k * 6 + d) * qcnt + qq] = sg[d].x;
-                    };
-                    for (int i = lane; i < npair * qcnt; i += TEAM) {
-                        const int k = i / qcnt, qq = i - k * qcnt, q = q0 + qq;
-                        const int k4 = ATT == ATT_CG4 ? cg4_slot(q) : q;
-                        T md[NM], dl = 0, dmu = 0;
-                        AT ds[6], mem[NSR][6];
-                        load_ops(k, q, k4, md, dl, dmu, ds, mem);
-                        // slices k and nr - k from one pass over the modes
-                        T Ac[6], Bc[6];
-#pragma unroll
-                        for (int d = 0; d < 6; d++) { Ac[d] = 0; Bc[d] = 0; }
-                        int j = 0;
-                        for (int al = 1; al < nu; al++) {
-                            j += k;
-                            j = j >= nr ? j - nr : j;
-                            const T2 w2 = tw2[j];
-#pragma unroll
-                            for (int d = 0; d < 6; d++) {
-                                const C ev = rA[(al * 6 + d) * 25 + q];
-                                Ac[d] += ev.x * w2.x;
-                                Bc[d] += ev.y * w2.y;
-                            }
-                        }
-                        T x1[6], x2[6];
-#pragma unroll
-                        for (int d = 0; d < 6; d++) {
-                            const T c0 = rA[d * 25 + q].x;
-                            x1[d] = c0 + (T)2 * (Ac[d] - Bc[d]);
-                            x2[d] = c0 + (T)2 * (Ac[d] + Bc[d]);
-                        }
-                        stress_slice(k, qq, k4, x1, md, dl, dmu, ds, mem);
-                        if (k != 0 && 2 * k != nr) {
-                            load_ops(nr - k, q, k4, md, dl, dmu, ds, mem);
-                            stress_slice(nr - k, qq, k4, x2, md, dl, dmu, ds, mem);
-                        }
-                    }
-                    team_sync(team, TEAM);
-                } else
-#endif
                 {
                 // Register-resident slice path. Two passes:
                 //  1. computeC2R, one thread per (slice pair, point): slices k and nr - k
@@ -1356,16 +788,10 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
                 //  2. one thread per (slice, point): the global operands of the point-slice
                 //     (moduli, attenuation moduli, SLS state) are loaded into registers,
                 //     stress and attenuation applied, the state stored back.
-#if AXG_SLICE_PAIRS
                 // KPc slice pairs per thread: each mode value read from shared memory feeds
                 // 2 KPc products
                 const int npair = nr / 2 + 1;
                 const int npb = (npair + KPc - 1) / KPc;
-#if AXG_TC_DFT
-                if (sizeof(T) == 4 && qcnt == 25) {
-                    tc_fourier_to_slices<T>(rA, rBr, sTws, nr, lane, TEAM);
-                } else
-#endif
 #if AXG_COLUMN_TILES
                 if (qcnt == 25) {
                     // column n = d * 25 + q of the block: mode a at rA[a * 150 + n], slice k
@@ -1460,11 +886,10 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
                     }
                 }
                 team_sync(team, TEAM);
-#endif
                 }
                 }   // direct Fourier -> slice sums
                 const int sp = use_fft ? 2 * vs.ps : 2 * qcnt, sq = use_fft ? 1 : qcnt;
-                for (int i = lane; i < (fused_done ? 0 : nr * qcnt); i += TEAM) {
+                for (int i = lane; i < nr * qcnt; i += TEAM) {
                     const int k = i / qcnt, qq = i - k * qcnt, q = q0 + qq;
                     T *slb = sl_base(k, qq);
                     T md[NM];
@@ -1485,49 +910,19 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
                             const T *am = a.attmod + a.att_off[e];
                             dl = __ldg(am + slot);
                             dmu = __ldg(am + nslot + slot);
-#if !AXG_SLS_SPLIT
-#if AXG_STATE_EARLY
-                            if (pre && i == lane) {
-#pragma unroll
-                                for (int d = 0; d < 6; d++) ds[d] = ds0[d];
-#pragma unroll
-                                for (int l = 0; l < NSR; l++)
-#pragma unroll
-                                    for (int d = 0; d < 6; d++) mem[l][d] = mem0[l][d];
-                            } else
-#endif
                             {
 #pragma unroll
-                            for (int d = 0; d < 6; d++) ds[d] = state_ld(st + d * nslot + slot);
+                            for (int d = 0; d < 6; d++) ds[d] = *(st + d * nslot + slot);
 #pragma unroll
                             for (int l = 0; l < NSR; l++)
 #pragma unroll
-                                for (int d = 0; d < 6; d++) mem[l][d] = state_ld(st + (6 + l * 6 + d) * nslot + slot);
+                                for (int d = 0; d < 6; d++) mem[l][d] = *(st + (6 + l * 6 + d) * nslot + slot);
                             }
-#endif
                         }
                     }
                     T acc[6];
-#if AXG_SLICE_PAIRS
 #pragma unroll
                     for (int d = 0; d < 6; d++) acc[d] = slb[(d >> 1) * sp + (d & 1) * sq];
-#else
-                    // computeC2R at slice k: r = Re c0 + 2 sum Re(c_a e^{i a phi_k})
-#pragma unroll
-                    for (int d = 0; d < 6; d++) acc[d] = rA[d * 25 + q].x;
-                    int j = 0;
-                    for (int al = 1; al < nu; al++) {
-                        j += k;
-                        j = j >= nr ? j - nr : j;
-                        const T2 w2 = tw2[j];
-                        const T c = w2.x, sn = w2.y;
-#pragma unroll
-                        for (int d = 0; d < 6; d++) {
-                            const C ev = rA[(al * 6 + d) * 25 + q];
-                            acc[d] += (T)2 * (ev.x * c - ev.y * sn);
-                        }
-                    }
-#endif
                     re1<T> ev[6], sg[6];
 #pragma unroll
                     for (int d = 0; d < 6; d++) ev[d].x = acc[d];
@@ -1543,22 +938,15 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
                             T e6[6], s6[6];
 #pragma unroll
                             for (int d = 0; d < 6; d++) { e6[d] = ev[d].x; s6[d] = sg[d].x; }
-#if AXG_SLS_SPLIT
-                            attenuate_slice_split<NSR, T, AT>(a.alpha, a.beta, a.gamma, st, nslot, slot, e6, s6, dl,
-                                                              dmu);
-#pragma unroll
-                            for (int d = 0; d < 6; d++) sg[d].x = s6[d];
-#else
                             attenuate_regs<NSR, T, AT>(a.alpha, a.beta, a.gamma, ds, mem, e6, s6, dl, dmu);
 #pragma unroll
                             for (int d = 0; d < 6; d++) sg[d].x = s6[d];
 #pragma unroll
-                            for (int d = 0; d < 6; d++) state_st(st + d * nslot + slot, ds[d]);
+                            for (int d = 0; d < 6; d++) *(st + d * nslot + slot) = ds[d];
 #pragma unroll
                             for (int l = 0; l < NSR; l++)
 #pragma unroll
-                                for (int d = 0; d < 6; d++) state_st(st + (6 + l * 6 + d) * nslot + slot, mem[l][d]);
-#endif
+                                for (int d = 0; d < 6; d++) *(st + (6 + l * 6 + d) * nslot + slot) = mem[l][d];
                         }
                     }
 #pragma unroll
@@ -1660,11 +1048,6 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
                     continue;
                 }
                 // slices -> Fourier (computeR2C) into region A for these points
-#if AXG_TC_DFT
-                if (!RTZ && sizeof(T) == 4 && qcnt == 25) {
-                    tc_slices_to_fourier<T>(rA, rBr, sTws, nr, inv_nr, lane, TEAM);
-                } else
-#endif
 #if AXG_COLUMN_TILES
                 if (!RTZ && qcnt == 25) {
                     // ABc modes x 6 columns per thread (the column layout of the Fourier ->

@@ -1,0 +1,81 @@
+"""Elements without 3-D properties run in tiles of modes (solid1d_kernel.cuh): parity with the FP64
+oracle at the edges of the tiles -- one mode, a full tile, one mode more, several uneven tiles --
+for the block sizes that axg_set_team_size allows, on the axis and off it, and with batched
+wavefields split over blocks.
+
+Tolerances: a force is a sum of about 1e2 products, each operand rounded once, so its relative
+2-norm error is a few units of the working precision: 2e-6 in float, 1e-13 in double.
+"""
+import numpy as np
+import pytest
+
+from axisem3d_b200 import meshgen
+from axisem3d_b200.solver import Solver
+
+pytestmark = pytest.mark.gpu
+
+TOL = {"fp32": 2e-6, "mixed": 2e-6, "fp64": 1e-13}
+
+
+def _oracle_steps(m, u, n):
+    import oracle as O
+    o = O.Oracle(m, "fp64", threads=4)
+    o.set_field(u, "displ")
+    o.compute_stiffness()
+    f = o.get_field("stiff")
+    o2 = O.Oracle(m, "fp64", threads=4)
+    o2.set_field(u, "displ")
+    o2.run(n)
+    return f, o2.get_field("displ")
+
+
+@pytest.mark.parametrize("precision", ["fp32", "mixed", "fp64"])
+@pytest.mark.parametrize("nrs", [[1], [1, 2, 3], [8, 9], [9, 10, 11], [20, 21], [63, 64]])
+@pytest.mark.parametrize("team", [0, 32, 256])
+def test_tiles_match_oracle(built, precision, nrs, team):
+    m = meshgen.microbench_model(n_elem=12, nr_choices=nrs, is3d=False, axial_column=True, seed=3)
+    u = meshgen.random_displacement(m, seed=4)
+    f, d = _oracle_steps(m, u, 4)
+    teams = {c: team for c in range(5)} if team else None
+    with Solver(m, precision, team_sizes=teams) as s:
+        s.set_field(u, "displ")
+        s.compute_stiffness()
+        g = s.get_field("stiff")
+        assert np.linalg.norm(g - f) <= TOL[precision] * np.linalg.norm(f)
+    with Solver(m, precision, team_sizes=teams) as s:
+        s.set_field(u, "displ")
+        s.run(4)
+        assert np.linalg.norm(s.get_field("displ") - d) <= TOL[precision] * np.linalg.norm(d)
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("nr", [1, 2, 9, 11, 12, 40])
+def test_cg4_tiles_match_oracle(built, precision, nr):
+    """CG4: the recursion runs on threads of its own, one per (component, attenuating slot)."""
+    m = meshgen.microbench_model(n_elem=9, nr_choices=[nr], is3d=False, rheology="iso", attenuation="cg4", seed=5)
+    u = meshgen.random_displacement(m, seed=6)
+    f, d = _oracle_steps(m, u, 5)
+    with Solver(m, precision) as s:
+        s.set_field(u, "displ")
+        s.run(5)
+        assert np.linalg.norm(s.get_field("displ") - d) <= TOL[precision] * np.linalg.norm(d)
+
+
+@pytest.mark.parametrize("nwave", [2, 7])
+def test_waves_split_over_blocks(built, nwave):
+    """Few elements and several wavefields: each wavefield equals its own run."""
+    m = meshgen.microbench_model(n_elem=4, nr_choices=[9, 11], is3d=False, seed=7)
+    us = [meshgen.random_displacement(m, seed=10 + w) for w in range(nwave)]
+    one = []
+    for u in us:
+        with Solver(m, "fp64") as s:
+            s.set_field(u, "displ")
+            s.run(5)
+            one.append(s.get_field("displ"))
+    m.nwave = nwave
+    with Solver(m, "fp64") as s:
+        s.set_field(np.concatenate(us), "displ")
+        s.run(5)
+        got = s.get_field("displ").reshape(nwave, -1)
+    for w in range(nwave):
+        assert np.linalg.norm(got[w] - one[w]) <= 1e-13 * np.linalg.norm(one[w])

@@ -55,6 +55,20 @@ struct DBuf {
     }
 };
 
+// Several buckets, several handles on one device and handles of different precision (the fluid
+// kernels of FP32 and mixed handles are the same functions) can share one kernel, and its dynamic
+// shared memory limit is an attribute of the function on that device, not of a handle: one record
+// for the whole process, in which the limit only ever rises.
+inline void raise_smem_limit(int device, const void *kernel, size_t bytes) {
+    static std::mutex mu;
+    static std::map<std::pair<int, const void *>, size_t> limits;
+    std::lock_guard<std::mutex> lock(mu);
+    size_t &cur = limits[{device, kernel}];
+    if (bytes <= cur) return;
+    AXG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    cur = bytes;
+}
+
 // team size per nr class and the nr class boundaries
 constexpr int kNrClasses = 5;
 inline int nr_class(int nr) { return nr <= 3 ? 0 : nr <= 9 ? 1 : nr <= 25 ? 2 : nr <= 64 ? 3 : 4; }
@@ -1506,18 +1520,7 @@ private:
         AXG_CUDA(cudaStreamSynchronize(stream_));
     }
 
-    // several buckets, and several handles on one device, can share one kernel instantiation,
-    // and its dynamic shared memory limit is an attribute of the function on that device, not of
-    // a handle: the limit only ever rises, to the largest any handle has asked for
-    void raise_smem_limit(const void *kernel, size_t bytes) {
-        static std::mutex mu;
-        static std::map<std::pair<int, const void *>, size_t> limits;
-        std::lock_guard<std::mutex> lock(mu);
-        size_t &cur = limits[{cfg_.device, kernel}];
-        if (bytes <= cur) return;
-        cur = bytes;
-        AXG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    }
+    void raise_smem_limit(const void *kernel, size_t bytes) { axg::raise_smem_limit(cfg_.device, kernel, bytes); }
 
     // ------------------------------------------------------- fluid buckets ---
     using FluidKernel = void (*)(const FluidArgs<T>, int, int, size_t);

@@ -79,3 +79,18 @@ def test_waves_split_over_blocks(built, nwave):
         got = s.get_field("displ").reshape(nwave, -1)
     for w in range(nwave):
         assert np.linalg.norm(got[w] - one[w]) <= 1e-13 * np.linalg.norm(one[w])
+
+
+def test_handles_of_two_precisions_share_kernels(built):
+    """FP32 and mixed handles launch the same fluid kernels: a small handle of one precision must
+    not lower the shared-memory limit that a large one of the other has raised."""
+    large = meshgen.spherical_model(n_theta=24, n_solid_layers=3, n_fluid_layers=1, nr_min=125, nr_max=125)
+    small = meshgen.spherical_model(n_theta=8, n_solid_layers=2, n_fluid_layers=1, nr_min=81, nr_max=81)
+    for precision, other in (("mixed", "fp32"), ("fp32", "mixed")):
+        with Solver(large, precision) as s:
+            s.run(2)
+        with Solver(small, other) as s:
+            s.run(2)
+        with Solver(large, precision) as s:
+            s.run(2)
+            assert np.all(np.isfinite(s.get_field("displ")))

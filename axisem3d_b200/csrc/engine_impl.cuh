@@ -72,9 +72,12 @@ inline void raise_smem_limit(int device, const void *kernel, size_t bytes) {
 // team size per nr class and the nr class boundaries
 constexpr int kNrClasses = 5;
 inline int nr_class(int nr) { return nr <= 3 ? 0 : nr <= 9 ? 1 : nr <= 25 ? 2 : nr <= 64 ? 3 : 4; }
-// smallest nr of a 3-D element that takes the slice FFTs instead of the direct sums (0 = never)
+// smallest nr of a 3-D element that takes the slice FFTs instead of the direct sums (0 = never):
+// from the nr class where the sums' nr^2 / 2 products per column outweigh two passes over shared
+// memory. Block meshes with nr up to 64 (FP32 / mixed, 20 steps): from 65 6.32 / 23.43 ms, from 26
+// 6.22 / 23.25, from 17 6.28 / 23.41.
 #ifndef AXG_FFT_MIN_NR
-#define AXG_FFT_MIN_NR 65
+#define AXG_FFT_MIN_NR 26
 #endif
 
 inline int default_team(int cls) {
@@ -233,6 +236,10 @@ public:
         std::vector<int> twoff;
         tw_.upload(twiddle_pool<T>(nrs, nrmax, twoff));
         tw_off_.upload(twoff);
+        std::vector<unsigned> plan(nrmax + 1, 0u);
+        if (AXG_FFT_MIN_NR > 0)
+            for (int n = AXG_FFT_MIN_NR; n <= nrmax; n++) plan[n] = fft_factors(n, fft_max_radix<T>());
+        fft_plan_.upload(plan);
         build_solid_buckets(m.se);
         build_fluid_buckets(m.fe);
         if (cfg_.autotune && !cfg_.plain) autotune();
@@ -1430,6 +1437,8 @@ private:
         }
         if (total > budget)
             throw Error(AXG_E_UNSUPPORTED, "SolidElement::expandWorkspace || nr too large for shared memory.");
+        const int qc1 = qc, mt1 = mt;
+        const size_t total1 = total;
 #if AXG_QC_FOR_TWO_CTAS
         // a one-element CTA too large for two per SM: smaller point chunks of the slice phase
         // often let a second CTA in
@@ -1468,6 +1477,19 @@ private:
             }
         }
 #endif
+        // Too large for two blocks per SM as it is: one block of 512 threads that keeps the whole
+        // chunk and all modes at once, rather than two of 256 with smaller chunks and tiles (more
+        // passes and barriers for the same registers). Measured on B200: shell with nr up to 128,
+        // CG4, 26.3 -> 23.0 ms for 20 steps; FP64 blocks with nr up to 64 16.2 -> 14.7 ms; where two
+        // whole elements fit, the 512-thread block is the slower one (FP32, nr up to 64: 6.2 -> 7.6 ms).
+        const bool dflt = !team_req && !cfg_.plain && !team_override_[b.cls];
+        if (dflt && team == 256 && !b.prt && (b.fft || sizeof(T) == 8) && total1 <= budget &&
+            total1 > (size_t)110 * 1024) {
+            qc = qc1;
+            mt = mt1;
+            total = total1;
+            team = 512;
+        }
         b.qc = qc;
         b.mt = mt;
         b.team_bytes = total;
@@ -2168,7 +2190,7 @@ private:
                                                                                b.team_bytes);
         } else {
             SolidArgs<T, AT> af = a;
-            af.fft_min_nr = b.fft ? AXG_FFT_MIN_NR : 0;
+            af.fft_plan = b.fft ? fft_plan_.p : nullptr;
             af.tab = b.tab.p;
             af.tiles = b.tiles.p;
             if (b.kernel1d) {
@@ -2518,6 +2540,7 @@ private:
     DBuf<int> er_elem_, er_gll_, er_kind_;
     DBuf<int64_t> er_off_;
     DBuf<C> er_out_;
+    DBuf<unsigned> fft_plan_;
     DBuf<int> step_dev_, nonfinite_;
 };
 

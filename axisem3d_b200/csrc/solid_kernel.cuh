@@ -18,7 +18,7 @@
 //   scatter-add: point.stiff -= f   SolidPoint::gatherStiffFromElement (SolidPoint.hpp:101-109)
 //
 // Shared memory per team (T = float or double, C = complex T):
-//   geometry 10 x 25 T, trig 4 x 25 T, point tables 3 x 25 int, twiddles 2 x nr T,
+//   geometry 10 x 25 T, trig 4 x 25 T, twiddles 2 x nr T,
 //   region A: 6 x nu x 25 C  (strain E, then stress S, then quadrature X/Y)
 //   region B: max(3 x mt x 25 C, nr x 6 x qc T)  (u, then stress slices, then A terms)
 // The gather + gradient and the two quadrature passes run over tiles of mt modes (each
@@ -27,6 +27,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "slice_fft.cuh"
 
 namespace axg {
 
@@ -103,7 +104,7 @@ struct SolidArgs {
     int nwave;                 // wavefields sharing the mesh (independent sources)
     size_t fstride;            // complex values between wavefields in displ / stiff
     size_t sstride;            // AT values between wavefields in the state pool
-    int fft_min_nr;            // 3-D elements with nr >= this (and 13-smooth nr) take the FFT; 0 = never
+    const unsigned *fft_plan;  // [nr_max + 1] radices of every nr that takes the FFT (fft_factors), 0 = direct sums
     const int2 *tab;           // [n][25] first mode and number of modes of the element's points
     const int4 *tiles;         // 1-D elements: (element, first mode, modes, nu | axial << 30) per block
 };
@@ -125,7 +126,6 @@ __host__ __device__ inline TeamLayout team_layout(int nr_max, int qc, int mt) {
     auto al = [](size_t x) { return (x + 15) & ~(size_t)15; };
     L.geom = o; o = al(o + 10 * 25 * sizeof(T));
     L.trig = o; o = al(o + 4 * 25 * sizeof(T));
-    L.ipt = o;  o = al(o + 3 * 25 * sizeof(int));
     L.tw = o;   o = al(o + 2 * (size_t)nr_max * sizeof(T));
     L.regA = o; o = al(o + 6 * (size_t)L.nu_max * 25 * 2 * sizeof(T));
     size_t b1 = 3 * (size_t)mt * 25 * 2 * sizeof(T);
@@ -388,177 +388,18 @@ __device__ __forceinline__ int cg4_slot(int q) {
     return q == 6 ? 0 : q == 8 ? 1 : q == 16 ? 2 : q == 18 ? 3 : -1;
 }
 
-// ------------------------------------------------------------- slice FFT ---
-// The phi transforms of a 3-D element (SolverFFTW::computeC2R / computeR2C, SolverFFTW.hpp:
-// 101-172: R2C scaled by 1/nr, the Nyquist mode halved, imaginary parts of modes 0 and nr/2
-// dropped; C2R with the Nyquist mode doubled) as complex FFTs of length nr over a batch of
-// S = 3 qc signals: the six strain / stress components of a point go in pairs, x_2p + i x_2p+1,
-// one complex signal per pair. The FFT is a mixed-radix Stockham transform in shared memory
-// (radices 4, 2, 3, 5, 7, 11, 13: every nr the reference's lucky-number rule admits), one pass
-// per radix between two buffers. Signal s = pair pp of
-// point qq of the chunk (s = pp qc + qq), sample n. The two buffers are views of shared memory
-// the element holds anyway: region B as [n][pp][qq] (row n of 3 qc values), and the columns of
-// the chunk's points in region A, whose strain the spectra were formed from and whose stress
-// the last pass's unpacking writes, as rows 3 n + pp of 25 values. Twiddles come from the
-// element's table of exp(2 pi i j / nr).
-
-// radices of n, powers of 4 first, then 2, 3, 5, 7, 11, 13, packed 3 bits per pass (codes
-// 1..7 for 4, 2, 3, 5, 7, 11, 13) into the returned plan; 0 if n has another prime factor
-// (those transforms take the direct sums)
-__device__ __forceinline__ unsigned fft_plan(int n) {
-    unsigned plan = 0;
-    int c = 0;
-    while (n % 4 == 0) { plan |= 1u << (3 * c++); n /= 4; }
-    while (n % 2 == 0) { plan |= 2u << (3 * c++); n /= 2; }
-    while (n % 3 == 0) { plan |= 3u << (3 * c++); n /= 3; }
-    while (n % 5 == 0) { plan |= 4u << (3 * c++); n /= 5; }
-    while (n % 7 == 0) { plan |= 5u << (3 * c++); n /= 7; }
-    while (n % 11 == 0) { plan |= 6u << (3 * c++); n /= 11; }
-    while (n % 13 == 0) { plan |= 7u << (3 * c++); n /= 13; }
-    return (n == 1 && c <= 10) ? plan : 0u;
-}
-
-// twiddle exp(sign 2 pi i m / N) from the interleaved (cos, sin) table
-template <class T>
-__device__ __forceinline__ cx_t<T> fft_tw(const cx_t<T> *tw2, int m, int sign) {
-    const cx_t<T> w = tw2[m];
-    return mk<T>(w.x, sign > 0 ? w.y : -w.y);
-}
-template <class T>
-__device__ __forceinline__ cx_t<T> cmul(cx_t<T> a, cx_t<T> b) {
-    return mk<T>(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-
-// in-register DFT of R points with sign: V_t = sum_r v_r exp(sign 2 pi i r t / R)
-template <int R, class T>
-__device__ __forceinline__ void fft_radix(cx_t<T> v[R], int sign, const cx_t<T> *tw2, int N) {
-    using C = cx_t<T>;
-    if constexpr (R == 2) {
-        const C a = v[0], b = v[1];
-        v[0] = cadd(a, b);
-        v[1] = csub(a, b);
-    } else if constexpr (R == 4) {
-        const C s02 = cadd(v[0], v[2]), d02 = csub(v[0], v[2]);
-        const C s13 = cadd(v[1], v[3]), d13 = csub(v[1], v[3]);
-        // j d13 with j = sign i
-        const C jd = sign > 0 ? mk<T>(-d13.y, d13.x) : mk<T>(d13.y, -d13.x);
-        v[0] = cadd(s02, s13);
-        v[2] = csub(s02, s13);
-        v[1] = cadd(d02, jd);
-        v[3] = csub(d02, jd);
-    } else {
-        C V[R];
-        const int step = N / R;
-#pragma unroll
-        for (int t = 0; t < R; t++) {
-            C acc = v[0];
-#pragma unroll
-            for (int r = 1; r < R; r++) acc = cadd(acc, cmul<T>(v[r], fft_tw<T>(tw2, ((r * t) % R) * step, sign)));
-            V[t] = acc;
-        }
-#pragma unroll
-        for (int t = 0; t < R; t++) v[t] = V[t];
-    }
-}
-
-// a batch of signals in shared memory: sample n of signal (pp, qq) at p[n rs + pp ps + qq]
-template <class T>
-struct FftView {
-    cx_t<T> *p;
-    int rs, ps;
-    __device__ __forceinline__ cx_t<T> &at(int n, int pp, int qq) const { return p[n * rs + pp * ps + qq]; }
-};
-
-// quotient of 0 <= x < 2^22 by d > 0, rd = 1 / d (the float quotient is off by at most one and
-// corrected): the index splits of the FFT passes without integer division
-__device__ __forceinline__ int div_n(int x, int d, float rd) {
-    int q = (int)((float)x * rd);
-    const int r = x - q * d;
-    q -= r < 0 ? 1 : 0;
-    q += r >= d ? 1 : 0;
-    return q;
-}
-
-// one Stockham pass of radix R over 3 qc signals: Ns = product of the earlier radices
-template <int R, class T>
-__device__ __forceinline__ void fft_pass_r(const FftView<T> in, const FftView<T> out, int N, int qc, int Ns,
-                                           int sign, const cx_t<T> *tw2, int lane, int TEAM) {
-    using C = cx_t<T>;
-    const int S = 3 * qc;
-    const int NR = N / R, span = N / (Ns * R);
-    const float rS = 1.f / (float)S, rNs = 1.f / (float)Ns;
-    for (int i = lane; i < NR * S; i += TEAM) {
-        const int j = div_n(i, S, rS), s = i - j * S;
-        const int pp = (s >= qc) + (s >= 2 * qc), qq = s - pp * qc;
-        const int jn = div_n(j, Ns, rNs), k = j - jn * Ns;
-        C v[R];
-#pragma unroll
-        for (int r = 0; r < R; r++) v[r] = in.at(j + r * NR, pp, qq);
-        const int step = k * span;
-        int m = 0;
-#pragma unroll
-        for (int r = 1; r < R; r++) {
-            m += step;
-            m = m >= N ? m - N : m;
-            if (step) v[r] = cmul<T>(v[r], fft_tw<T>(tw2, m, sign));
-        }
-        const int d = jn * Ns * R + k;
-        if constexpr (R >= 11) {
-            // the larger primes: each output summed and stored in turn (fewer live registers)
-            const int stepR = N / R;
-#pragma unroll 1
-            for (int t = 0; t < R; t++) {
-                C acc = v[0];
-                int m2 = 0;
-#pragma unroll
-                for (int r = 1; r < R; r++) {
-                    m2 += t;
-                    m2 = m2 >= R ? m2 - R : m2;
-                    acc = cadd(acc, cmul<T>(v[r], fft_tw<T>(tw2, m2 * stepR, sign)));
-                }
-                out.at(d + t * Ns, pp, qq) = acc;
-            }
-        } else {
-            fft_radix<R, T>(v, sign, tw2, N);
-#pragma unroll
-            for (int r = 0; r < R; r++) out.at(d + r * Ns, pp, qq) = v[r];
-        }
-    }
-}
-
-// the whole transform of the 3 qc signals of length N from view b0 by the packed plan, passes
-// alternating between b0 and b1; returns the view that holds the result (natural order); the
-// team synchronises after every pass
-template <class T>
-__device__ __forceinline__ FftView<T> fft_run(FftView<T> b0, FftView<T> b1, int N, int qc, unsigned plan,
-                                              int sign, const cx_t<T> *tw2, int team, int lane, int TEAM) {
-    FftView<T> in = b0, out = b1;
-    int Ns = 1;
-    for (; plan; plan >>= 3) {
-        int R;
-        switch (plan & 7u) {
-            case 1: fft_pass_r<4, T>(in, out, N, qc, Ns, sign, tw2, lane, TEAM); R = 4; break;
-            case 2: fft_pass_r<2, T>(in, out, N, qc, Ns, sign, tw2, lane, TEAM); R = 2; break;
-            case 3: fft_pass_r<3, T>(in, out, N, qc, Ns, sign, tw2, lane, TEAM); R = 3; break;
-            case 4: fft_pass_r<5, T>(in, out, N, qc, Ns, sign, tw2, lane, TEAM); R = 5; break;
-            case 5: fft_pass_r<7, T>(in, out, N, qc, Ns, sign, tw2, lane, TEAM); R = 7; break;
-            case 6: fft_pass_r<11, T>(in, out, N, qc, Ns, sign, tw2, lane, TEAM); R = 11; break;
-            default: fft_pass_r<13, T>(in, out, N, qc, Ns, sign, tw2, lane, TEAM); R = 13; break;
-        }
-        team_sync(team, TEAM);
-        Ns *= R;
-        const FftView<T> t = in; in = out; out = t;
-    }
-    return in;
-}
-
 // ----------------------------------------------------------------- kernel ---
+// Largest block: 512 threads where an element can be too large for two blocks per SM (FP64, and
+// the large nr of the FFT instantiations), so that the one block still fills the register file.
+template <class T, bool FFT>
+constexpr int solid_threads() { return FFT || sizeof(T) == 8 ? 512 : 256; }
+
 // NS: compile-time number of SLS for the register-resident recursion; 0 = the generic path with
 // the count read at run time
 // FFT: the instantiation that holds the slice FFTs (buckets with large nr); the others
 // keep only the direct sums, so the FFT code costs them no registers
 template <class T, class AT, int RHEO, int ATT, bool RTZ, int NS, bool FFT = false>
-__global__ void __launch_bounds__(256, AXG_SOLID_MIN_BLOCKS)
+__global__ void __launch_bounds__(solid_threads<T, FFT>(), solid_threads<T, FFT>() == 512 ? 1 : AXG_SOLID_MIN_BLOCKS)
 solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_max, const int mt_max,
                        const int teams_per_cta, const size_t team_bytes) {
     using C = cx_t<T>;
@@ -582,9 +423,6 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
     unsigned char *base = smem_raw + (size_t)team * team_bytes;
     T *sGeo = reinterpret_cast<T *>(base + L.geom);
     T *sTrig = reinterpret_cast<T *>(base + L.trig);
-    int *sPt = reinterpret_cast<int *>(base + L.ipt);
-    int *sOff = sPt + 25;
-    int *sNu = sPt + 50;
     T *sTw = reinterpret_cast<T *>(base + L.tw);
     C *rA = reinterpret_cast<C *>(base + L.regA);
     C *rBc = reinterpret_cast<C *>(base + L.regB);
@@ -606,21 +444,15 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
         for (int i = lane; i < 250; i += TEAM) sGeo[i] = a.geom[(size_t)e * 250 + i];
         if constexpr (RTZ)
             for (int i = lane; i < 100; i += TEAM) sTrig[i] = a.trig[(size_t)e * 100 + i];
-        for (int i = lane; i < 25; i += TEAM) {
-            int p = a.pts[(size_t)e * 25 + i];
-            sPt[i] = p;
-            sOff[i] = a.pt_off[p];
-            sNu[i] = a.pt_nu[p];
-        }
+        const int2 *tab = a.tab + (size_t)e * 25;
         {
             const T *tw = a.tw + a.tw_off[nr];
             // interleaved (cos, sin) pairs: one 2-word shared load per twiddle
             for (int i = lane; i < 2 * nr; i += TEAM) sTw[i] = (i & 1) ? tw[nr + (i >> 1)] : tw[i >> 1];
         }
-        team_sync(team, TEAM);
-
-        // every wavefield of the batch reuses the element header loaded above
-        for (int w = 0; w < a.nwave; w++) {
+        // every wavefield of the batch reuses the element header; the barrier after the first gather
+        // covers it
+        for (int w = blockIdx.y; w < a.nwave; w += gridDim.y) {
         const C *displw = a.displ + (size_t)w * a.fstride;
         C *stiffw = a.stiff + (size_t)w * a.fstride;
         AT *statew = a.state + (size_t)w * a.sstride;
@@ -629,11 +461,13 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
         for (int t0 = 0; t0 < nu; t0 += mt_max) {
         const int mt = min(mt_max, nu - t0);
         // ---------------- gather displacement: U[a - t0][c][q] in region B ----------------
+        const float rmt = 1.f / (float)mt;
         for (int i = lane; i < mt * 25; i += TEAM) {
-            const int q = i / mt, la = i - q * mt, al = t0 + la;
+            const int q = div_n(i, mt, rmt), la = i - q * mt, al = t0 + la;
+            const int2 on = __ldg(tab + q);
             C u0 = mk<T>(0, 0), u1 = u0, u2 = u0;
-            if (al < sNu[q]) {
-                const C *src = displw + (size_t)(sOff[q] + al) * 3;
+            if (al < on.y) {
+                const C *src = displw + ((size_t)on.x + al) * 3;
                 u0 = src[0]; u1 = src[1]; u2 = src[2];
             }
             rBc[(la * 3 + 0) * 25 + q] = u0;
@@ -663,47 +497,22 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
                 X[c] = x; Y[c] = y;
             }
             const T ze = dzdeta[q], zx = dzdxii[q], se = dsdeta[q], sx = dsdxii[q];
-            C eps[6];
-            // dS/dZ of u0 -> e0, e4 ; u1 -> e5, e3 ; u2 -> e1, e2
-            eps[0] = cadd(cscale(X[0], ze), cscale(Y[0], zx));
-            eps[4] = cadd(cscale(X[0], se), cscale(Y[0], sx));
-            eps[5] = cadd(cscale(X[1], ze), cscale(Y[1], zx));
+            C eps[6], S[3];
+#pragma unroll
+            for (int c = 0; c < 3; c++) S[c] = cadd(cscale(X[c], ze), cscale(Y[c], zx));
+            eps[0] = S[0];
+            eps[4] = cadd(cadd(cscale(X[0], se), cscale(Y[0], sx)), S[2]);
             eps[3] = cadd(cscale(X[1], se), cscale(Y[1], sx));
-            C e1t = cadd(cscale(X[2], ze), cscale(Y[2], zx));
             eps[2] = cadd(cscale(X[2], se), cscale(Y[2], sx));
-            eps[4] = cadd(eps[4], e1t);
-            // lower-order terms A/s
+            // lower-order terms A / s; on the axis (L'Hopital) dA / ds, the same combination of
+            // the derivatives
             const T alf = (T)al;
-            const C u0 = U[q], u1 = U[25 + q], u2 = U[50 + q];
-            const C A0 = csub(cia(alf, u0), u1);
-            const C A1 = cadd(cia(alf, u1), u0);
-            const C A2 = cia(alf, u2);
-            const T is = invs[q];
-            eps[5] = cadd(eps[5], cscale(A0, is));
-            eps[1] = cscale(A1, is);
-            eps[3] = cadd(eps[3], cscale(A2, is));
-            if (axial && ii == 0) {
-                // L'Hopital on the axis: row 0 of A/s replaced by dA/ds
-                C ax[3], ay[3];
-#pragma unroll
-                for (int c = 0; c < 3; c++) { ax[c] = mk<T>(0, 0); ay[c] = mk<T>(0, 0); }
-#pragma unroll
-                for (int k = 0; k < 5; k++) {
-                    const T gx = Gxi[k * 5 + 0];
-                    const T gy = sGll[k * 5 + jj];
-                    const C v0 = U[k * 5 + jj], v1 = U[25 + k * 5 + jj], v2 = U[50 + k * 5 + jj];
-                    const C w0 = U[k], w1 = U[25 + k], w2 = U[50 + k];
-                    C a0 = csub(cia(alf, v0), v1), a1 = cadd(cia(alf, v1), v0), a2 = cia(alf, v2);
-                    C b0 = csub(cia(alf, w0), w1), b1 = cadd(cia(alf, w1), w0), b2 = cia(alf, w2);
-                    ax[0] = cadd(ax[0], cscale(a0, gx)); ax[1] = cadd(ax[1], cscale(a1, gx));
-                    ax[2] = cadd(ax[2], cscale(a2, gx));
-                    ay[0] = cadd(ay[0], cscale(b0, gy)); ay[1] = cadd(ay[1], cscale(b1, gy));
-                    ay[2] = cadd(ay[2], cscale(b2, gy));
-                }
-                eps[5] = cadd(eps[5], cadd(cscale(ax[0], ze), cscale(ay[0], zx)));
-                eps[1] = cadd(cscale(ax[1], ze), cscale(ay[1], zx));
-                eps[3] = cadd(eps[3], cadd(cscale(ax[2], ze), cscale(ay[2], zx)));
-            }
+            const bool lim = axial && ii == 0;
+            const C b0 = lim ? S[0] : U[q], b1 = lim ? S[1] : U[25 + q], b2 = lim ? S[2] : U[50 + q];
+            const T is = lim ? (T)1 : invs[q];
+            eps[5] = cadd(S[1], cscale(csub(cia(alf, b0), b1), is));
+            eps[1] = cscale(cadd(cia(alf, b1), b0), is);
+            eps[3] = cadd(eps[3], cscale(cia(alf, b2), is));
             if constexpr (RTZ) {
                 spz_to_rtz6(eps, sTrig[q], sTrig[25 + q], sTrig[50 + q], sTrig[75 + q]);
             }
@@ -737,7 +546,7 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
             // the FFT path (register-resident slice path only): an nr the plan covers
             unsigned plan = 0;
             if constexpr (FFT && (NS > 0 || ATT == ATT_NONE)) {
-                if (a.fft_min_nr > 0 && nr >= a.fft_min_nr) plan = fft_plan(nr);
+                if (a.fft_plan) plan = __ldg(a.fft_plan + nr);
             }
             const bool use_fft = FFT && plan != 0;
             for (int q0 = 0; q0 < 25; q0 += qc_max) {
@@ -745,11 +554,7 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
                 // slices of this chunk: [k][d][qq] reals in region B (direct sums) or, on the
                 // FFT path, x_2p + i x_2p+1 of sample k in whichever view the C2R left them
                 const FftView<T> vB{rBc, 3 * qcnt, qcnt}, vA{rA + q0, 75, 25};
-                FftView<T> vs = vB;
-                // component d of slice k at point qq: base(k, qq) + (d >> 1) sp + (d & 1) sq
-                auto sl_base = [&](int k, int qq) -> T * {
-                    return use_fft ? reinterpret_cast<T *>(&vs.at(k, 0, qq)) : rBr + (size_t)k * 6 * qcnt + qq;
-                };
+                FftView<T> vs = vB, vo = vB;   // strain slices, stress slices
                 if constexpr (NS > 0 || ATT == ATT_NONE) {
                 constexpr int NM = RHEO == RHEO_ISO ? 2 : RHEO == RHEO_TISO ? 5 : 21;
                 constexpr int NSR = NS > 0 ? NS : 1;
@@ -757,26 +562,11 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
                 const T *modp = a.mod + moff;
                 const size_t nsl = (size_t)nslice * 25;
                 if (FFT && use_fft) {
-                    // Hermitian spectra of the component pairs, Z = Y_2p + i Y_2p+1 over all nr
-                    // orders: Y_0 = Re c_0, Y_a = c_a, Y_nr-a = conj c_a, Y_nr/2 = 2 Re c_nr/2
-                    for (int i = lane; i < (nr / 2 + 1) * qcnt; i += TEAM) {
-                        const int al = i / qcnt, qq = i - al * qcnt, q = q0 + qq;
-#pragma unroll
-                        for (int pp = 0; pp < 3; pp++) {
-                            const C c1 = rA[(al * 6 + 2 * pp) * 25 + q], c2 = rA[(al * 6 + 2 * pp + 1) * 25 + q];
-                            if (al == 0) {
-                                vB.at(0, pp, qq) = mk<T>(c1.x, c2.x);
-                            } else if (2 * al == nr) {
-                                vB.at(al, pp, qq) = mk<T>((T)2 * c1.x, (T)2 * c2.x);
-                            } else {
-                                vB.at(al, pp, qq) = mk<T>(c1.x - c2.y, c1.y + c2.x);
-                                vB.at(nr - al, pp, qq) = mk<T>(c1.x + c2.y, c2.x - c1.y);
-                            }
-                        }
-                    }
-                    team_sync(team, TEAM);
-                    // from here on the chunk's columns of region A are free until the unpacking
-                    vs = fft_run<T>(vB, vA, nr, qcnt, plan, +1, tw2, team, lane, TEAM);
+                    // from here on the chunk's columns of region A are free until the unpacking; the
+                    // stress goes to the view the strain is not in, from which the passes back end
+                    // in region B
+                    vs = fft_run<T>(rA + q0, vA, vB, nr, qcnt, plan, tw2, team, lane, TEAM);
+                    vo = vs.p == rBc ? vA : vB;
                 } else {
                 {
                 // Register-resident slice path. Two passes:
@@ -888,10 +678,15 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
                 team_sync(team, TEAM);
                 }
                 }   // direct Fourier -> slice sums
+                // component d of slice k at point qq: in + (d >> 1) sp + (d & 1) sq, and the stress at
+                // out + (d >> 1) op + (d & 1) oq (the FFT takes its pairs with the parts exchanged)
                 const int sp = use_fft ? 2 * vs.ps : 2 * qcnt, sq = use_fft ? 1 : qcnt;
-                for (int i = lane; i < nr * qcnt; i += TEAM) {
-                    const int k = i / qcnt, qq = i - k * qcnt, q = q0 + qq;
-                    T *slb = sl_base(k, qq);
+                const int op = use_fft ? 2 * vo.ps : 2 * qcnt, oq = use_fft ? -1 : qcnt;
+                auto stress_at = [&](int k, int qq, auto with_att) {
+                    constexpr bool ATTEN = decltype(with_att)::value;
+                    const int q = q0 + qq;
+                    const T *in = use_fft ? reinterpret_cast<const T *>(&vs.at(k, 0, qq)) : rBr + (size_t)k * 6 * qcnt + qq;
+                    T *out = use_fft ? reinterpret_cast<T *>(&vo.at(k, 0, qq)) + 1 : rBr + (size_t)k * 6 * qcnt + qq;
                     T md[NM];
 #pragma unroll
                     for (int mm = 0; mm < NM; mm++) md[mm] = __ldg(modp + mm * nsl + (size_t)k * 25 + q);
@@ -899,33 +694,23 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
                     T dl = 0, dmu = 0;
                     AT *st = nullptr;
                     size_t slot = 0, nslot = 0;
-                    bool att_here = false;
-                    if constexpr (ATT != ATT_NONE) {
-                        const int k4 = ATT == ATT_CG4 ? cg4_slot(q) : q;
-                        att_here = k4 >= 0;
-                        if (att_here) {
-                            nslot = (size_t)nr * NPA;
-                            slot = (size_t)k * NPA + k4;
-                            st = statew + a.state_off[e];
-                            const T *am = a.attmod + a.att_off[e];
-                            dl = __ldg(am + slot);
-                            dmu = __ldg(am + nslot + slot);
-                            {
+                    if constexpr (ATTEN) {
+                        nslot = (size_t)nr * NPA;
+                        slot = (size_t)k * NPA + (ATT == ATT_CG4 ? cg4_slot(q) : q);
+                        st = statew + a.state_off[e];
+                        const T *am = a.attmod + a.att_off[e];
+                        dl = __ldg(am + slot);
+                        dmu = __ldg(am + nslot + slot);
 #pragma unroll
-                            for (int d = 0; d < 6; d++) ds[d] = *(st + d * nslot + slot);
+                        for (int d = 0; d < 6; d++) ds[d] = st[d * nslot + slot];
 #pragma unroll
-                            for (int l = 0; l < NSR; l++)
+                        for (int l = 0; l < NSR; l++)
 #pragma unroll
-                                for (int d = 0; d < 6; d++) mem[l][d] = *(st + (6 + l * 6 + d) * nslot + slot);
-                            }
-                        }
+                            for (int d = 0; d < 6; d++) mem[l][d] = st[(6 + l * 6 + d) * nslot + slot];
                     }
-                    T acc[6];
-#pragma unroll
-                    for (int d = 0; d < 6; d++) acc[d] = slb[(d >> 1) * sp + (d & 1) * sq];
                     re1<T> ev[6], sg[6];
 #pragma unroll
-                    for (int d = 0; d < 6; d++) ev[d].x = acc[d];
+                    for (int d = 0; d < 6; d++) ev[d].x = in[(d >> 1) * sp + (d & 1) * sq];
                     if constexpr (RHEO == RHEO_ISO) {
                         stress_iso(ev, sg, md[0], md[1]);
                     } else if constexpr (RHEO == RHEO_TISO) {
@@ -933,24 +718,42 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
                     } else {
                         stress_aniso(ev, sg, md);
                     }
-                    if constexpr (ATT != ATT_NONE) {
-                        if (att_here) {
-                            T e6[6], s6[6];
+                    if constexpr (ATTEN) {
+                        T e6[6], s6[6];
 #pragma unroll
-                            for (int d = 0; d < 6; d++) { e6[d] = ev[d].x; s6[d] = sg[d].x; }
-                            attenuate_regs<NSR, T, AT>(a.alpha, a.beta, a.gamma, ds, mem, e6, s6, dl, dmu);
+                        for (int d = 0; d < 6; d++) { e6[d] = ev[d].x; s6[d] = sg[d].x; }
+                        attenuate_regs<NSR, T, AT>(a.alpha, a.beta, a.gamma, ds, mem, e6, s6, dl, dmu);
 #pragma unroll
-                            for (int d = 0; d < 6; d++) sg[d].x = s6[d];
+                        for (int d = 0; d < 6; d++) sg[d].x = s6[d];
 #pragma unroll
-                            for (int d = 0; d < 6; d++) *(st + d * nslot + slot) = ds[d];
+                        for (int d = 0; d < 6; d++) st[d * nslot + slot] = ds[d];
 #pragma unroll
-                            for (int l = 0; l < NSR; l++)
+                        for (int l = 0; l < NSR; l++)
 #pragma unroll
-                                for (int d = 0; d < 6; d++) *(st + (6 + l * 6 + d) * nslot + slot) = mem[l][d];
-                        }
+                            for (int d = 0; d < 6; d++) st[(6 + l * 6 + d) * nslot + slot] = mem[l][d];
                     }
 #pragma unroll
-                    for (int d = 0; d < 6; d++) slb[(d >> 1) * sp + (d & 1) * sq] = sg[d].x;
+                    for (int d = 0; d < 6; d++) out[(d >> 1) * op + (d & 1) * oq] = sg[d].x;
+                };
+                if constexpr (ATT == ATT_CG4) {
+                    // the four attenuating points apart from the elastic ones, so that no warp
+                    // runs the recursion for a few of its lanes: c0 of them lie before the chunk
+                    auto before = [](int q) { return (q > 6) + (q > 8) + (q > 16) + (q > 18); };
+                    const int c0 = before(q0), nc = before(q0 + qcnt) - c0, ne = qcnt - nc;
+                    const float rne = 1.f / (float)max(ne, 1);
+                    for (int i = lane; i < nr * nc; i += TEAM) {
+                        const int k = nc == 4 ? i >> 2 : i / nc, k4 = c0 + i - k * nc;
+                        stress_at(k, 6 + 2 * (k4 & 1) + 10 * (k4 >> 1) - q0, std::true_type{});
+                    }
+                    for (int i = lane; i < nr * ne; i += TEAM) {
+                        const int k = div_n(i, ne, rne), j = q0 - c0 + i - k * ne;
+                        stress_at(k, j + (j >= 6) + (j >= 7) + (j >= 14) + (j >= 15) - q0, std::false_type{});
+                    }
+                } else {
+                    for (int i = lane; i < nr * qcnt; i += TEAM) {
+                        const int k = i / qcnt;
+                        stress_at(k, i - k * qcnt, std::integral_constant<bool, ATT != ATT_NONE>{});
+                    }
                 }
                 } else
                 // Fourier -> slices (computeC2R), stress, attenuation -> rBr[k][d][qq]
@@ -1020,9 +823,7 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
                 if (FFT && use_fft) {
                     // forward FFT of the stress pairs, then each pair's two spectra:
                     // S_2p = (Z_a + conj Z_nr-a) / 2, S_2p+1 = (Z_a - conj Z_nr-a) / 2i, scaled by 1/nr
-                    // an even number of passes in all: the spectra end in region B, and the
-                    // unpacking below writes the chunk's columns of region A without a race
-                    const FftView<T> Z = fft_run<T>(vs, vs.p == rBc ? vA : vB, nr, qcnt, plan, -1, tw2, team, lane, TEAM);
+                    const FftView<T> Z = fft_run<T>(nullptr, vo, vs, nr, qcnt, plan, tw2, team, lane, TEAM);
                     const T h = (T)0.5 * inv_nr;
                     for (int i = lane; i < nu * qcnt; i += TEAM) {
                         const int al = i / qcnt, qq = i - al * qcnt, q = q0 + qq;
@@ -1030,7 +831,8 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
                         C sg[6];
 #pragma unroll
                         for (int pp = 0; pp < 3; pp++) {
-                            const C za = Z.at(al, pp, qq), zb = Z.at(bl, pp, qq);
+                            const C ya = Z.at(al, pp, qq), yb = Z.at(bl, pp, qq);
+                            const C za = mk<T>(ya.y, ya.x), zb = mk<T>(yb.y, yb.x);   // parts back in place
                             T r1 = (za.x + zb.x) * h, m1 = (za.y - zb.y) * h;
                             T r2 = (za.y + zb.y) * h, m2 = (zb.x - za.x) * h;
                             if (al == 0) { m1 = 0; m2 = 0; }
@@ -1170,67 +972,85 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
         for (int t0 = 0; t0 < nu; t0 += mt_max) {
         const int mt = min(mt_max, nu - t0);
         // ---------------- quadrature (computeQuad6), pass 1: X, Y, A ----------------
+        // the axial terms (the transpose of dA / ds) join X and Y at the axial row
         for (int i = lane; i < mt * 25; i += TEAM) {
             const int la = i / 25, q = i - la * 25, al = t0 + la;
             C s[6];
 #pragma unroll
             for (int d = 0; d < 6; d++) s[d] = rA[(al * 6 + d) * 25 + q];
             const T ze = dzdeta_if[q], zx = dzdxii_if[q], se = dsdeta_if[q], sx = dsdxii_if[q];
+            const T alf = (T)al, is = invs_if[q];
+            C A[3], x[6];
+            A[0] = csub(cia(alf, s[5]), s[1]);
+            A[1] = cadd(cia(alf, s[1]), s[5]);
+            A[2] = cia(alf, s[3]);
+            x[0] = cadd(cscale(s[0], ze), cscale(s[4], se));
+            x[1] = cadd(cscale(s[0], zx), cscale(s[4], sx));
+            x[2] = cadd(cscale(s[5], ze), cscale(s[3], se));
+            x[3] = cadd(cscale(s[5], zx), cscale(s[3], sx));
+            x[4] = cadd(cscale(s[4], ze), cscale(s[2], se));
+            x[5] = cadd(cscale(s[4], zx), cscale(s[2], sx));
+            if (axial && q < 5) {
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    x[2 * c] = csub(x[2 * c], cscale(A[c], ze));
+                    x[2 * c + 1] = csub(x[2 * c + 1], cscale(A[c], zx));
+                }
+            }
             C *xy = rA + al * 150;
-            xy[0 * 25 + q] = cadd(cscale(s[0], ze), cscale(s[4], se));
-            xy[1 * 25 + q] = cadd(cscale(s[0], zx), cscale(s[4], sx));
-            xy[2 * 25 + q] = cadd(cscale(s[5], ze), cscale(s[3], se));
-            xy[3 * 25 + q] = cadd(cscale(s[5], zx), cscale(s[3], sx));
-            xy[4 * 25 + q] = cadd(cscale(s[4], ze), cscale(s[2], se));
-            xy[5 * 25 + q] = cadd(cscale(s[4], zx), cscale(s[2], sx));
-            const T alf = (T)al;
-            rBc[(la * 3 + 0) * 25 + q] = csub(cia(alf, s[5]), s[1]);
-            rBc[(la * 3 + 1) * 25 + q] = cadd(cia(alf, s[1]), s[5]);
-            rBc[(la * 3 + 2) * 25 + q] = cia(alf, s[3]);
+#pragma unroll
+            for (int d = 0; d < 6; d++) xy[d * 25 + q] = x[d];
+#pragma unroll
+            for (int c = 0; c < 3; c++) rBc[(la * 3 + c) * 25 + q] = cscale(A[c], is);
         }
         team_sync(team, TEAM);
 
-        // ---------------- quadrature pass 2 + scatter-add ----------------
+        // ---------------- quadrature pass 2: the forces, in the place of A ----------------
         for (int i = lane; i < mt * 25; i += TEAM) {
             const int la = i / 25, q = i - la * 25, al = t0 + la;
             const int ii = q / 5, jj = q - ii * 5;
             const C *xy = rA + al * 150;
-            const C *A = rBc + la * 75;
+            C *A = rBc + la * 75 + q;
             C f[3];
 #pragma unroll
-            for (int c = 0; c < 3; c++) {
-                C g1 = mk<T>(0, 0), g2 = mk<T>(0, 0);
+            for (int c = 0; c < 3; c++) f[c] = mk<T>(-A[c * 25].x, -A[c * 25].y);
 #pragma unroll
-                for (int k = 0; k < 5; k++) {
-                    const T gx = Gxi[ii * 5 + k];      // G_xi(ii, k)
-                    const T gt = sGll[jj * 5 + k];     // GT_GLL(k, jj) = G_GLL(jj, k)
+            for (int k = 0; k < 5; k++) {
+                const T gx = Gxi[ii * 5 + k];      // G_xi(ii, k)
+                const T gt = sGll[jj * 5 + k];     // GT_GLL(k, jj) = G_GLL(jj, k)
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
                     const C xv = xy[(2 * c) * 25 + k * 5 + jj];
                     const C yv = xy[(2 * c + 1) * 25 + ii * 5 + k];
-                    g1.x += gx * xv.x; g1.y += gx * xv.y;
-                    g2.x += yv.x * gt; g2.y += yv.y * gt;
+                    f[c].x += gx * xv.x; f[c].y += gx * xv.y;
+                    f[c].x += yv.x * gt; f[c].y += yv.y * gt;
                 }
-                C fc = cadd(g1, g2);
-                fc = csub(fc, cscale(A[c * 25 + q], invs_if[q]));
-                if (axial) {
-                    const T g0 = Gxi[ii * 5 + 0];
-                    fc = csub(fc, cscale(cscale(A[c * 25 + jj], dzdeta_if[jj]), g0));
-                    if (ii == 0) {
-                        C b = mk<T>(0, 0);
-#pragma unroll
-                        for (int k = 0; k < 5; k++) {
-                            const C y0 = cscale(A[c * 25 + k], dzdxii_if[k]);
-                            const T gt = sGll[jj * 5 + k];
-                            b.x += y0.x * gt; b.y += y0.y * gt;
-                        }
-                        fc = csub(fc, b);
-                    }
-                }
-                f[c] = fc;
             }
-            if (al < sNu[q]) {
-                C *dst = stiffw + (size_t)(sOff[q] + al) * 3;
+            if constexpr (sizeof(T) == 4) {
+                // scatter-add, one vector reduction per component
+                const int2 on = __ldg(tab + q);
+                if (al < on.y) {
+                    C *dst = stiffw + ((size_t)on.x + al) * 3;
 #pragma unroll
-                for (int c = 0; c < 3; c++) atomic_add_cx(dst + c, mk<T>(-f[c].x, -f[c].y));
+                    for (int c = 0; c < 3; c++) atomic_add_cx(dst + c, mk<T>(-f[c].x, -f[c].y));
+                }
+            } else {
+#pragma unroll
+                for (int c = 0; c < 3; c++) A[c * 25] = f[c];
+            }
+        }
+        if constexpr (sizeof(T) == 8) {
+            // FP64 has no vector reduction: the forces go through shared memory, so that a warp's
+            // lanes cover consecutive words of the field (point, mode, component, part)
+            team_sync(team, TEAM);
+            const int run = 6 * mt;
+            const float rrun = 1.f / (float)run;
+            for (int j = lane; j < 25 * run; j += TEAM) {
+                const int p = div_n(j, run, rrun), r = j - p * run;
+                const int2 on = __ldg(tab + p);
+                const T f = reinterpret_cast<const T *>(rBc + (r >> 1) * 25 + p)[r & 1];
+                if (t0 + r / 6 < on.y)
+                    atomicAdd(reinterpret_cast<T *>(stiffw + ((size_t)on.x + t0) * 3) + r, -f);
             }
         }
         team_sync(team, TEAM);

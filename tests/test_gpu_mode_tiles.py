@@ -94,3 +94,40 @@ def test_handles_of_two_precisions_share_kernels(built):
         with Solver(large, precision) as s:
             s.run(2)
             assert np.all(np.isfinite(s.get_field("displ")))
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("nrs", [
+    [26, 27], [28, 30, 32], [33, 35, 36], [39, 40, 42, 44], [45, 48, 49, 50], [52, 54, 55, 56], [60, 63, 64, 65],
+    [66, 70, 72, 75, 77], [78, 80, 81, 84, 88], [90, 91, 96, 98, 99], [100, 104, 105, 108, 110],
+    [112, 117, 120, 121], [125, 126, 128], [29, 31, 34, 37, 58, 61]])
+@pytest.mark.parametrize("attenuation", [None, "full"])
+def test_slice_transforms_match_oracle(built, precision, nrs, attenuation):
+    """3-D elements of every nr from 26 on: FFTs where nr has no prime factor above 13 (every radix
+    and every pair of radices of two-pass transforms, three passes), direct sums for the others."""
+    m = meshgen.microbench_model(n_elem=9, nr_choices=nrs, rheology="iso", attenuation=attenuation, seed=nrs[0])
+    u = meshgen.random_displacement(m, seed=8)
+    f, d = _oracle_steps(m, u, 3)
+    with Solver(m, precision) as s:
+        s.set_field(u, "displ")
+        s.compute_stiffness()
+        g = s.get_field("stiff")
+        assert np.linalg.norm(g - f) <= TOL[precision] * np.linalg.norm(f)
+    with Solver(m, precision) as s:
+        s.set_field(u, "displ")
+        s.run(3)
+        assert np.linalg.norm(s.get_field("displ") - d) <= TOL[precision] * np.linalg.norm(d)
+
+
+@pytest.mark.parametrize("nr", [26, 100])
+def test_cg4_slices_match_oracle(built, nr):
+    """CG4 on slices: the attenuating points run apart from the elastic ones, also where a chunk of
+    the slice phase holds only some of them."""
+    m = meshgen.microbench_model(n_elem=6, nr_choices=[nr], attenuation="cg4", seed=9)
+    u = meshgen.random_displacement(m, seed=8)
+    f, d = _oracle_steps(m, u, 4)
+    for teams in (None, {3: 128, 4: 128}):
+        with Solver(m, "mixed", team_sizes=teams) as s:
+            s.set_field(u, "displ")
+            s.run(4)
+            assert np.linalg.norm(s.get_field("displ") - d) <= TOL["mixed"] * np.linalg.norm(d)

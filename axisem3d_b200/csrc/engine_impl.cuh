@@ -784,8 +784,8 @@ public:
             a.fstride = 0;
             a.x = b.xpool.p; a.x_off = b.xoff.p; a.x3d = b.x3d.p; a.trig = b.trig.p;
             int blocks = (b.n + b.tpc - 1) / b.tpc;
-            b.kernel<<<blocks, b.team * b.tpc, b.tpc * b.team_bytes, ls()>>>(a, b.nr_max, b.tpc,
-                                                                              b.team_bytes);
+            b.kernel<<<wave_grid(blocks, a.nwave), b.team * b.tpc, b.tpc * b.team_bytes, ls()>>>(a, b.nr_max, b.tpc,
+                                                                                              b.team_bytes);
             post_launch();
         });
         // one after another where the sums must come in one order
@@ -1404,9 +1404,9 @@ private:
     }
     // wavefields of a batch on (y, z) of the grid: split over blocks while the elements alone do
     // not fill the GPU several times over (each split loads the element's operands again)
-    dim3 wave_grid(int blocks) const {
+    dim3 wave_grid(int blocks, int nwave) const {
         const int want = std::max(1, prop_.multiProcessorCount * 16 / std::max(blocks, 1));
-        return dim3((unsigned)blocks, (unsigned)std::min({nwave_, want, 65535}), 1);
+        return dim3((unsigned)blocks, (unsigned)std::min({nwave, want, 65535}), 1);
     }
 
     void configure_bucket(SolidBucket &b, int team_req = 0) {
@@ -2193,13 +2193,10 @@ private:
             af.fft_plan = b.fft ? fft_plan_.p : nullptr;
             af.tab = b.tab.p;
             af.tiles = b.tiles.p;
-            if (b.kernel1d) {
-                dim3 g = wave_grid(b.grid);
-                g.y = std::min(g.y, (unsigned)a.nwave);
-                b.kernel1d<<<g, b.team, b.team_bytes, ls()>>>(af, b.mt);
-            } else
-            b.kernel<<<b.grid, b.team * b.tpc, b.tpc * b.team_bytes, ls()>>>(af, b.nr_max, b.qc, b.mt, b.tpc,
-                                                                              b.team_bytes);
+            const dim3 g = wave_grid(b.grid, a.nwave);
+            if (b.kernel1d) b.kernel1d<<<g, b.team, b.team_bytes, ls()>>>(af, b.mt);
+            else
+                b.kernel<<<g, b.team * b.tpc, b.tpc * b.team_bytes, ls()>>>(af, b.nr_max, b.qc, b.mt, b.tpc, b.team_bytes);
         }
         post_launch();
     }
@@ -2215,8 +2212,8 @@ private:
             a.fstride = (size_t)fp_.total;
             a.x = b.xpool.p; a.x_off = b.xoff.p; a.x3d = b.x3d.p; a.trig = b.trig.p;
             int blocks = (b.n + b.tpc - 1) / b.tpc;
-            b.kernel<<<blocks, b.team * b.tpc, b.tpc * b.team_bytes, ls()>>>(a, b.nr_max, b.tpc,
-                                                                              b.team_bytes);
+            b.kernel<<<wave_grid(blocks, a.nwave), b.team * b.tpc, b.tpc * b.team_bytes, ls()>>>(a, b.nr_max, b.tpc,
+                                                                                              b.team_bytes);
             post_launch();
         }
     }
@@ -2260,7 +2257,7 @@ private:
         a.s_displ = elem_displ(sp_); a.s_stiff = sp_.stiff.p; a.f_stiff = fp_.stiff.p;
         a.nwave = nwave_; a.s_stride = (size_t)sp_.total * 3; a.f_stride = (size_t)fp_.total;
         int threads = 256, blocks = (cp_n_ * 32 + threads - 1) / threads;
-        solid_fluid_kernel<T><<<blocks, threads, 0, ls()>>>(a);
+        solid_fluid_kernel<T><<<wave_grid(blocks, nwave_), threads, 0, ls()>>>(a);
         post_launch();
     }
 

@@ -146,7 +146,7 @@ fluid_stiffness_kernel(const FluidArgs<T> a, const int nr_max, const int teams_p
             for (int i = lane; i < 2 * nr; i += TEAM) sTw[i] = tw[i];
         }
         team_sync(team, TEAM);
-        for (int w = 0; w < a.nwave; w++) {
+        for (int w = blockIdx.y; w < a.nwave; w += gridDim.y) {
         const C *displw = a.displ + (size_t)w * a.fstride;
         C *stiffw = a.stiff + (size_t)w * a.fstride;
         for (int i = lane; i < nu * 25; i += TEAM) {

@@ -44,7 +44,7 @@ __global__ void solid_fluid_kernel(const CouplingArgs<T> a) {
     const int s = a.sp[pair], f = a.fp[pair];
     const int nu = a.f_nu[f];
     const T nsu = a.nsu[pair], nzu = a.nzu[pair], nsa = a.nsa_m[pair], nza = a.nza_m[pair];
-    for (int w = 0; w < a.nwave; w++) {
+    for (int w = blockIdx.y; w < a.nwave; w += gridDim.y) {
         const cx_t<T> *sd = a.s_displ + (size_t)w * a.s_stride;
         cx_t<T> *sst = a.s_stiff + (size_t)w * a.s_stride;
         cx_t<T> *fst = a.f_stiff + (size_t)w * a.f_stride;

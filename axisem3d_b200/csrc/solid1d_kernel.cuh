@@ -160,7 +160,7 @@ solid_1d_kernel(const SolidArgs<T, AT> a, const int mt_max) {
     }
     const T *Gl = a.gmat, *Gx = a.gmat + (axial ? 25 : 0);
 
-    for (int w = blockIdx.z * gridDim.y + blockIdx.y; w < a.nwave; w += gridDim.y * gridDim.z) {
+    for (int w = blockIdx.y; w < a.nwave; w += gridDim.y) {
         const C *displw = a.displ + (size_t)w * a.fstride;
         C *stiffw = a.stiff + (size_t)w * a.fstride;
         AT *st = ATT == ATT_NONE ? nullptr : a.state + (size_t)w * a.sstride + a.state_off[e];

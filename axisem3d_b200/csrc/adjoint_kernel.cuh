@@ -137,53 +137,34 @@ __device__ __forceinline__ void strain_at(const cx_t<T> *U, int al, int q, bool 
     const T *dsdxii = geo, *dsdeta = geo + 25, *dzdxii = geo + 50, *dzdeta = geo + 75, *invs = geo + 100;
     C X[3], Y[3];
 #pragma unroll
-    for (int c = 0; c < 3; c++) {
-        C x = mk<T>(0, 0), y = mk<T>(0, 0);
+    for (int c = 0; c < 3; c++) { X[c] = mk<T>(0, 0); Y[c] = mk<T>(0, 0); }
 #pragma unroll
-        for (int k = 0; k < 5; k++) {
-            const T gx = Gxi[k * 5 + ii], gy = sGll[k * 5 + jj];
+    for (int k = 0; k < 5; k++) {
+        const T gx = Gxi[k * 5 + ii], gy = sGll[k * 5 + jj];
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
             const C uc = U[c * 25 + k * 5 + jj], ur = U[c * 25 + ii * 5 + k];
-            x.x += gx * uc.x; x.y += gx * uc.y;
-            y.x += ur.x * gy; y.y += ur.y * gy;
+            X[c].x += gx * uc.x; X[c].y += gx * uc.y;
+            Y[c].x += ur.x * gy; Y[c].y += ur.y * gy;
         }
-        X[c] = x; Y[c] = y;
     }
     const T ze = dzdeta[q], zx = dzdxii[q], se = dsdeta[q], sx = dsdxii[q];
-    eps[0] = cadd(cscale(X[0], ze), cscale(Y[0], zx));
-    eps[4] = cadd(cscale(X[0], se), cscale(Y[0], sx));
-    eps[5] = cadd(cscale(X[1], ze), cscale(Y[1], zx));
+    C Sd[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) Sd[c] = cadd(cscale(X[c], ze), cscale(Y[c], zx));
+    eps[0] = Sd[0];
+    eps[4] = cadd(cadd(cscale(X[0], se), cscale(Y[0], sx)), Sd[2]);
     eps[3] = cadd(cscale(X[1], se), cscale(Y[1], sx));
-    const C e1t = cadd(cscale(X[2], ze), cscale(Y[2], zx));
     eps[2] = cadd(cscale(X[2], se), cscale(Y[2], sx));
-    eps[4] = cadd(eps[4], e1t);
+    // lower-order terms A / s; on the axis (L'Hopital) dA / ds, the same combination of the
+    // derivatives
     const T alf = (T)al;
-    const C A0 = csub(cia(alf, U[q]), U[25 + q]);
-    const C A1 = cadd(cia(alf, U[25 + q]), U[q]);
-    const C A2 = cia(alf, U[50 + q]);
-    const T is = invs[q];
-    eps[5] = cadd(eps[5], cscale(A0, is));
-    eps[1] = cscale(A1, is);
-    eps[3] = cadd(eps[3], cscale(A2, is));
-    if (axial && ii == 0) {
-        C ax[3], ay[3];
-#pragma unroll
-        for (int c = 0; c < 3; c++) { ax[c] = mk<T>(0, 0); ay[c] = mk<T>(0, 0); }
-#pragma unroll
-        for (int k = 0; k < 5; k++) {
-            const T gx = Gxi[k * 5 + 0], gy = sGll[k * 5 + jj];
-            const C v0 = U[k * 5 + jj], v1 = U[25 + k * 5 + jj], v2 = U[50 + k * 5 + jj];
-            const C w0 = U[k], w1 = U[25 + k], w2 = U[50 + k];
-            C a0 = csub(cia(alf, v0), v1), a1 = cadd(cia(alf, v1), v0), a2 = cia(alf, v2);
-            C b0 = csub(cia(alf, w0), w1), b1 = cadd(cia(alf, w1), w0), b2 = cia(alf, w2);
-            ax[0] = cadd(ax[0], cscale(a0, gx)); ax[1] = cadd(ax[1], cscale(a1, gx));
-            ax[2] = cadd(ax[2], cscale(a2, gx));
-            ay[0] = cadd(ay[0], cscale(b0, gy)); ay[1] = cadd(ay[1], cscale(b1, gy));
-            ay[2] = cadd(ay[2], cscale(b2, gy));
-        }
-        eps[5] = cadd(eps[5], cadd(cscale(ax[0], ze), cscale(ay[0], zx)));
-        eps[1] = cadd(cscale(ax[1], ze), cscale(ay[1], zx));
-        eps[3] = cadd(eps[3], cadd(cscale(ax[2], ze), cscale(ay[2], zx)));
-    }
+    const bool lim = axial && ii == 0;
+    const C b0 = lim ? Sd[0] : U[q], b1 = lim ? Sd[1] : U[25 + q], b2 = lim ? Sd[2] : U[50 + q];
+    const T is = lim ? (T)1 : invs[q];
+    eps[5] = cadd(Sd[1], cscale(csub(cia(alf, b0), b1), is));
+    eps[1] = cscale(cadd(cia(alf, b1), b0), is);
+    eps[3] = cadd(eps[3], cscale(cia(alf, b2), is));
 }
 
 // one CTA (team of blockDim.x threads) per element: -K g scattered to `out`, and the
@@ -194,7 +175,7 @@ __device__ __forceinline__ void strain_at(const cx_t<T> *U, int al, int q, bool 
 // sensitivities per element at mod_off / grad_off, RTZ frames); the isotropic one keeps its
 // lambda / mu layout. GENERIC is not combined with SLICES.
 template <class T, bool SLICES, bool GENERIC = false>
-__global__ void __launch_bounds__(256) adjoint_stiffness_kernel(const AdjointArgs<T> a, const int nu_max) {
+__global__ void __launch_bounds__(128, GENERIC ? 2 : 4) adjoint_stiffness_kernel(const AdjointArgs<T> a, const int nu_max) {
     static_assert(!(SLICES && GENERIC), "per-slice sensitivities are isotropic only");
     using C = cx_t<T>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -382,51 +363,63 @@ __global__ void __launch_bounds__(256) adjoint_stiffness_kernel(const AdjointArg
 #pragma unroll
             for (int d = 0; d < 6; d++) s[d] = S[(al * 6 + d) * 25 + q];
             const T ze = dzdeta_if[q], zx = dzdxii_if[q], se = dsdeta_if[q], sx = dsdxii_if[q];
+            const T alf = (T)al, is = invs_if[q];
+            C A[3], x[6];
+            A[0] = csub(cia(alf, s[5]), s[1]);
+            A[1] = cadd(cia(alf, s[1]), s[5]);
+            A[2] = cia(alf, s[3]);
+            x[0] = cadd(cscale(s[0], ze), cscale(s[4], se));
+            x[1] = cadd(cscale(s[0], zx), cscale(s[4], sx));
+            x[2] = cadd(cscale(s[5], ze), cscale(s[3], se));
+            x[3] = cadd(cscale(s[5], zx), cscale(s[3], sx));
+            x[4] = cadd(cscale(s[4], ze), cscale(s[2], se));
+            x[5] = cadd(cscale(s[4], zx), cscale(s[2], sx));
+            if (axial && q < 5) {
+                // the axial terms join X and Y at the axial row
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    x[2 * c] = csub(x[2 * c], cscale(A[c], ze));
+                    x[2 * c + 1] = csub(x[2 * c + 1], cscale(A[c], zx));
+                }
+            }
             C *xy = S + al * 150;
-            xy[0 * 25 + q] = cadd(cscale(s[0], ze), cscale(s[4], se));
-            xy[1 * 25 + q] = cadd(cscale(s[0], zx), cscale(s[4], sx));
-            xy[2 * 25 + q] = cadd(cscale(s[5], ze), cscale(s[3], se));
-            xy[3 * 25 + q] = cadd(cscale(s[5], zx), cscale(s[3], sx));
-            xy[4 * 25 + q] = cadd(cscale(s[4], ze), cscale(s[2], se));
-            xy[5 * 25 + q] = cadd(cscale(s[4], zx), cscale(s[2], sx));
-            const T alf = (T)al;
-            Ug[(al * 3 + 0) * 25 + q] = csub(cia(alf, s[5]), s[1]);
-            Ug[(al * 3 + 1) * 25 + q] = cadd(cia(alf, s[1]), s[5]);
-            Ug[(al * 3 + 2) * 25 + q] = cia(alf, s[3]);
+#pragma unroll
+            for (int d = 0; d < 6; d++) xy[d * 25 + q] = x[d];
+#pragma unroll
+            for (int c = 0; c < 3; c++) Ug[(al * 3 + c) * 25 + q] = cscale(A[c], is);
         }
         __syncthreads();
         for (int i = threadIdx.x; i < nu * 25; i += blockDim.x) {
             const int al = i / 25, q = i - al * 25;
             const int ii = q / 5, jj = q - ii * 5;
             const C *xy = S + al * 150;
-            const C *A = Ug + al * 75;
+            C *A = Ug + al * 75 + q;
+            C f[3];
 #pragma unroll
-            for (int c = 0; c < 3; c++) {
-                C g1 = mk<T>(0, 0), g2 = mk<T>(0, 0);
+            for (int c = 0; c < 3; c++) f[c] = mk<T>(-A[c * 25].x, -A[c * 25].y);
 #pragma unroll
-                for (int k = 0; k < 5; k++) {
-                    const T gx = Gxi[ii * 5 + k], gt = sGll[jj * 5 + k];
+            for (int k = 0; k < 5; k++) {
+                const T gx = Gxi[ii * 5 + k], gt = sGll[jj * 5 + k];
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
                     const C xv = xy[(2 * c) * 25 + k * 5 + jj], yv = xy[(2 * c + 1) * 25 + ii * 5 + k];
-                    g1.x += gx * xv.x; g1.y += gx * xv.y;
-                    g2.x += yv.x * gt; g2.y += yv.y * gt;
+                    f[c].x += gx * xv.x; f[c].y += gx * xv.y;
+                    f[c].x += yv.x * gt; f[c].y += yv.y * gt;
                 }
-                C fc = cadd(g1, g2);
-                fc = csub(fc, cscale(A[c * 25 + q], invs_if[q]));
-                if (axial) {
-                    fc = csub(fc, cscale(cscale(A[c * 25 + jj], dzdeta_if[jj]), Gxi[ii * 5 + 0]));
-                    if (ii == 0) {
-                        C b = mk<T>(0, 0);
-#pragma unroll
-                        for (int k = 0; k < 5; k++) {
-                            const C y0 = cscale(A[c * 25 + k], dzdxii_if[k]);
-                            const T gt = sGll[jj * 5 + k];
-                            b.x += y0.x * gt; b.y += y0.y * gt;
-                        }
-                        fc = csub(fc, b);
-                    }
-                }
-                if (al < sNu[q]) atomic_add_cx(a.out + (size_t)(sOff[q] + al) * 3 + c, mk<T>(-fc.x, -fc.y));
             }
+#pragma unroll
+            for (int c = 0; c < 3; c++) A[c * 25] = f[c];
+        }
+        __syncthreads();
+        // scatter-add of reals in the order of the field (point, mode, component, part): a warp's
+        // lanes cover consecutive words, where one FP64 reduction per lane and part covered a
+        // 32-byte sector each
+        const int run = 6 * nu;
+        const float rrun = 1.f / (float)run;
+        for (int j = threadIdx.x; j < 25 * run; j += blockDim.x) {
+            const int p = div_n(j, run, rrun), r = j - p * run;
+            const T f = reinterpret_cast<const T *>(Ug + (r >> 1) * 25 + p)[r & 1];
+            if (r / 6 < sNu[p]) atomicAdd(reinterpret_cast<T *>(a.out + (size_t)sOff[p] * 3) + r, -f);
         }
         }
         __syncthreads();

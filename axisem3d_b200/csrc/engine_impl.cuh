@@ -684,7 +684,7 @@ public:
                 }
                 const int nu_max = adj_nr_max_ / 2 + 1;
                 const size_t smem = (size_t)nu_max * (75 + 75 + 150 + (adj_slices_ ? 300 : 0)) * sizeof(C);
-                const int grid = std::min(model_.se.count, prop_.multiProcessorCount * 8);
+                const int grid = model_.se.count;   // a block per element: the scheduler refills an SM as any ends
                 if (adj_slices_) adjoint_stiffness_kernel<T, true><<<grid, 128, smem, stream_>>>(aa, nu_max);
                 else if (adj_generic_) adjoint_stiffness_kernel<T, false, true><<<grid, 128, smem, stream_>>>(aa, nu_max);
                 else adjoint_stiffness_kernel<T, false><<<grid, 128, smem, stream_>>>(aa, nu_max);

@@ -48,6 +48,8 @@ struct DBuf {
         n = count;
         if (count) AXG_CUDA(cudaMalloc(&p, count * sizeof(X)));
     }
+    // the buffer as it is when it has this size already
+    void fit(size_t count) { if (count != n || !p) alloc(count); }
     void zero(cudaStream_t s) { if (n) AXG_CUDA(cudaMemsetAsync(p, 0, n * sizeof(X), s)); }
     void upload(const std::vector<X> &h) {
         alloc(h.size());
@@ -535,8 +537,8 @@ public:
         ensure_capacity(step_ + nsteps);
         const size_t nf = (size_t)sp_.total * 3;
         const int nck = (nsteps + interval - 1) / interval;
-        ck_displ_.alloc(nf * nck); ck_veloc_.alloc(nf * nck); ck_accel_.alloc(nf * nck);
-        if (state_wave_ > 0) ck_state_.alloc((size_t)state_wave_ * nck);
+        ck_displ_.fit(nf * nck); ck_veloc_.fit(nf * nck); ck_accel_.fit(nf * nck);
+        if (state_wave_ > 0) ck_state_.fit((size_t)state_wave_ * nck);
         ck_n_ = nsteps; ck_interval_ = interval; ck_step0_ = step_;
         for (int c = 0; c < nck; c++) {
             copy_fields_out(c);
@@ -556,9 +558,27 @@ public:
         const size_t nf = (size_t)sp_.total * 3;
         const int nck = (ck_n_ + ck_interval_ - 1) / ck_interval_;
         const int end_step = ck_step0_ + ck_n_;
+        // the sweep's fields in one allocation (a dozen of them, the two segments the bulk, took
+        // longer to allocate and free than a short sweep to run), given back at the end
+        struct Part {
+            C *p = nullptr;
+        } fin_d, fin_v, fin_a, ub, vb, ab, g, gw, kt, seg_u, seg_a;
+        const size_t nfp = (nf + 15) / 16 * 16;
+        std::vector<std::pair<Part *, size_t>> parts;
+        for (Part *q : {&fin_d, &fin_v, &fin_a, &ub, &vb, &ab, &g}) parts.push_back({q, nfp});
+        if (adj_3d_)   // W^-1 g and the forward kernels' -K W^-1 g
+            for (Part *q : {&gw, &kt}) parts.push_back({q, nfp});
+        for (Part *q : {&seg_u, &seg_a}) parts.push_back({q, (nf * std::min(ck_interval_, ck_n_) + 15) / 16 * 16});
+        size_t words = 0;
+        for (auto &q : parts) words += q.second;
+        DBuf<C> work;
+        work.alloc(words);
+        words = 0;
+        for (auto &q : parts) {
+            q.first->p = work.p + words;
+            words += q.second;
+        }
         // state after the forward run, restored at the end
-        DBuf<C> fin_d, fin_v, fin_a;
-        fin_d.alloc(nf); fin_v.alloc(nf); fin_a.alloc(nf);
         AXG_CUDA(cudaMemcpyAsync(fin_d.p, sp_.displ.p, nf * sizeof(C), cudaMemcpyDeviceToDevice, stream_));
         AXG_CUDA(cudaMemcpyAsync(fin_v.p, sp_.veloc.p, nf * sizeof(C), cudaMemcpyDeviceToDevice, stream_));
         AXG_CUDA(cudaMemcpyAsync(fin_a.p, sp_.accel.p, nf * sizeof(C), cudaMemcpyDeviceToDevice, stream_));
@@ -569,14 +589,8 @@ public:
                                      stream_));
         }
         if (adj_astate_n_ > 0) adj_astate_.zero(stream_);
-        DBuf<C> ub, vb, ab, g, seg_u, seg_a, gw, kt;
-        ub.alloc(nf); vb.alloc(nf); ab.alloc(nf); g.alloc(nf);
-        ub.zero(stream_); vb.zero(stream_); ab.zero(stream_);
-        if (adj_3d_) {   // W^-1 g and the forward kernels' -K W^-1 g
-            gw.alloc(nf); kt.alloc(nf);
-            kt.zero(stream_);
-        }
-        seg_u.alloc(nf * ck_interval_); seg_a.alloc(nf * ck_interval_);
+        for (Part *q : {&ub, &vb, &ab}) AXG_CUDA(cudaMemsetAsync(q->p, 0, nf * sizeof(C), stream_));
+        if (adj_3d_) AXG_CUDA(cudaMemsetAsync(kt.p, 0, nf * sizeof(C), stream_));
         adj_grad_.zero(stream_);
         adj_gmass_.zero(stream_);
         if (adj_slices_) {
@@ -699,22 +713,20 @@ public:
             }
         }
         AXG_CUDA(cudaStreamSynchronize(stream_));
+        // (only FP64 handles come here: the caller's doubles are the device's)
         auto d2h_cx = [&](const C *src, double *dst) {
-            std::vector<C> hbuf(nf);
-            AXG_CUDA(cudaMemcpy(hbuf.data(), src, nf * sizeof(C), cudaMemcpyDeviceToHost));
-            for (size_t i = 0; i < nf; i++) { dst[2 * i] = (double)hbuf[i].x; dst[2 * i + 1] = (double)hbuf[i].y; }
+            if constexpr (std::is_same<T, double>::value)
+                AXG_CUDA(cudaMemcpy(dst, src, nf * sizeof(C), cudaMemcpyDeviceToHost));
         };
         if (grad_u0) d2h_cx(ub.p, grad_u0);
         if (grad_v0) d2h_cx(vb.p, grad_v0);
         if (grad_mod) {
-            std::vector<T> hg((size_t)adj_grad_n_);
-            AXG_CUDA(cudaMemcpy(hg.data(), adj_grad_.p, hg.size() * sizeof(T), cudaMemcpyDeviceToHost));
-            for (size_t i = 0; i < hg.size(); i++) grad_mod[i] = (double)hg[i];
+            if constexpr (std::is_same<T, double>::value)
+                AXG_CUDA(cudaMemcpy(grad_mod, adj_grad_.p, (size_t)adj_grad_n_ * sizeof(T), cudaMemcpyDeviceToHost));
         }
         if (grad_mass) {
-            std::vector<T> hm(sp_.n);
-            AXG_CUDA(cudaMemcpy(hm.data(), adj_gmass_.p, hm.size() * sizeof(T), cudaMemcpyDeviceToHost));
-            for (int i = 0; i < sp_.n; i++) grad_mass[i] = (double)hm[i];
+            if constexpr (std::is_same<T, double>::value)
+                AXG_CUDA(cudaMemcpy(grad_mass, adj_gmass_.p, (size_t)sp_.n * sizeof(T), cudaMemcpyDeviceToHost));
         }
         // back to the state after the forward run
         AXG_CUDA(cudaMemcpyAsync(sp_.displ.p, fin_d.p, nf * sizeof(C), cudaMemcpyDeviceToDevice, stream_));

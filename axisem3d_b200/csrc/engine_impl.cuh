@@ -191,7 +191,7 @@ public:
         for (int i = 0; i < kNrClasses; i++) team_override_[i] = 0;
     }
     ~Engine() override {
-        if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
+        drop_graphs();
         if (ev0_) cudaEventDestroy(ev0_);
         if (ev1_) cudaEventDestroy(ev1_);
         if (fork_ev_) cudaEventDestroy(fork_ev_);
@@ -303,8 +303,18 @@ public:
                 time_n_ += 1;
             }
         } else if (graph && !cfg_.plain) {
-            if (!graph_exec_) capture();
-            for (int i = 0; i < nsteps; i++) {
+            // several steps in one graph while there are enough of them: a graph's start and end
+            // cost a small mesh's step about as much as one of its kernels
+            int i = 0;
+            if (nsteps >= 2 * kGraphSteps) {
+                if (!graph_multi_) capture(graph_multi_, kGraphSteps);
+                for (; i + kGraphSteps <= nsteps; i += kGraphSteps) {
+                    AXG_CUDA(cudaGraphLaunch(graph_multi_, stream_));
+                    launches_ += kernels_per_step_ * kGraphSteps;
+                }
+            }
+            if (i < nsteps && !graph_exec_) capture(graph_exec_, 1);
+            for (; i < nsteps; i++) {
                 AXG_CUDA(cudaGraphLaunch(graph_exec_, stream_));
                 launches_ += kernels_per_step_;
             }
@@ -462,7 +472,7 @@ public:
         er_out_.zero(stream_);
         if (n) upload_elem_tables(grad);
         AXG_CUDA(cudaStreamSynchronize(stream_));
-        if (graph_exec_) { cudaGraphExecDestroy(graph_exec_); graph_exec_ = nullptr; }
+        drop_graphs();
     }
     int64_t element_record_words() const override { return er_words_; }
     void get_element_records(int rec_first, int nrec, double *out) override {
@@ -486,7 +496,7 @@ public:
     int64_t launches() const override { return launches_; }
     void set_timing(bool on) override {
         timing_ = on;
-        if (graph_exec_) { cudaGraphExecDestroy(graph_exec_); graph_exec_ = nullptr; }
+        drop_graphs();
         time_ms_ = 0; time_n_ = 0;
     }
     void stiffness_time(double *ms, int64_t *n) override {
@@ -519,7 +529,7 @@ public:
     void set_stream(void *s) override {
         stream_ = s ? (cudaStream_t)s : own_stream_;
         dev_step_ = -1;   // set again in the new stream's order
-        if (graph_exec_) { cudaGraphExecDestroy(graph_exec_); graph_exec_ = nullptr; }
+        drop_graphs();
     }
     void set_team_override(int cls, int team) override {
         if (cls < 0 || cls >= kNrClasses) throw Error(AXG_E_ARG, "Engine::set_team_override || bad class");
@@ -615,7 +625,7 @@ public:
             dev_step_ = -1;
             // recompute the segment, keeping u_n and a_n (the forward step's graph, which reads
             // the step from the device counter set above)
-            if (!cfg_.plain && !graph_exec_) capture();
+            if (!cfg_.plain && !graph_exec_) capture(graph_exec_, 1);
             for (int i = 0; i < len; i++) {
                 AXG_CUDA(cudaMemcpyAsync(seg_u.p + nf * i, sp_.displ.p, nf * sizeof(C),
                                          cudaMemcpyDeviceToDevice, stream_));
@@ -1996,7 +2006,7 @@ private:
                 changed = true;
             }
         }
-        if (changed && graph_exec_) { cudaGraphExecDestroy(graph_exec_); graph_exec_ = nullptr; }
+        if (changed) drop_graphs();
     }
     static T src_stf(const HostSources &h, int i, double t) {
         auto it = h.table.find(i);
@@ -2434,20 +2444,28 @@ private:
             throw Error(AXG_E_CUDA, std::string("Engine::launch || ") + cudaGetErrorString(e));
     }
 
-    void capture() {
+    static constexpr int kGraphSteps = 8;
+    void drop_graphs() {
+        for (cudaGraphExec_t *e : {&graph_exec_, &graph_multi_}) {
+            if (*e) cudaGraphExecDestroy(*e);
+            *e = nullptr;
+        }
+    }
+    // `steps` time steps, which read and advance the device step counter, as one graph
+    void capture(cudaGraphExec_t &exec, int steps) {
         cudaGraph_t g;
         int64_t before = launches_;
         AXG_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
         try {
-            launch_step();
+            for (int i = 0; i < steps; i++) launch_step();
         } catch (...) {
             cudaStreamEndCapture(stream_, &g);
             throw;
         }
         AXG_CUDA(cudaStreamEndCapture(stream_, &g));
-        kernels_per_step_ = launches_ - before;
+        kernels_per_step_ = (launches_ - before) / steps;
         launches_ = before;
-        AXG_CUDA(cudaGraphInstantiate(&graph_exec_, g, 0));
+        AXG_CUDA(cudaGraphInstantiate(&exec, g, 0));
         cudaGraphDestroy(g);
     }
 
@@ -2467,7 +2485,7 @@ private:
     double time_ms_ = 0;
     int64_t time_n_ = 0;
     cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;
-    cudaGraphExec_t graph_exec_ = nullptr;
+    cudaGraphExec_t graph_exec_ = nullptr, graph_multi_ = nullptr;   // one step, kGraphSteps steps
     int team_override_[kNrClasses];
     struct Tuned { int cls, team; float ms; };
     std::vector<Tuned> tuned_;

@@ -656,7 +656,9 @@ __global__ void __launch_bounds__(POINT_BLOCK) point_update_kernel(const PointAr
     const bool update = (a.mask & 4) != 0;
     const uint8_t fl = a.mode_flags[mm];
     const T inv = a.mode_inv[mm];
-    cx_t<T> f = a.stiff[q], acc = mk<T>(0, 0);
+    // the boundary stage on its own leaves most modes as they are: those are not touched
+    const bool touch = a.mask != 1 || (fl & (MODE_AXIS0 | MODE_AXIS1 | MODE_ZERO | MODE_NYQUIST)) != 0;
+    cx_t<T> f = touch ? a.stiff[q] : mk<T>(0, 0), acc = mk<T>(0, 0);
     cx_t<D> v = mk<D>(0, 0), u = v;
     cx_t<float> cv = mk<float>(0, 0), cd = cv;
     if (update) {
@@ -673,7 +675,7 @@ __global__ void __launch_bounds__(POINT_BLOCK) point_update_kernel(const PointAr
         g1 = a.stiff[q - d + 1];
     }
     __syncthreads();
-    if (!valid) return;
+    if (!valid || !touch) return;
     if (!(fl & MODE_SKIP)) {
         if (a.mask & 1) {
             // point_bc for one component

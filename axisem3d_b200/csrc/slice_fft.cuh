@@ -112,11 +112,12 @@ __device__ __forceinline__ void fft_dft(cx_t<T> (&v)[R]) {
             fft_for<H>([&](auto j) {
                 constexpr int k = (decltype(j)::value + 1) * (decltype(t)::value + 1) % R;
                 constexpr T c = (T)fft_cos(2 * k, R), s = (T)fft_sin(2 * k, R);
-                m.x += c * a[j].x; m.y += c * a[j].y;
-                n.x += s * b[j].x; n.y += s * b[j].y;
+                m = cmac(m, a[j], c);
+                n = cmac(n, b[j], s);
             });
-            v[t + 1] = mk<T>(m.x - n.y, m.y + n.x);
-            v[R - 1 - t] = mk<T>(m.x + n.y, m.y - n.x);
+            const C jn = mk<T>(-n.y, n.x);
+            v[t + 1] = cadd(m, jn);
+            v[R - 1 - t] = csub(m, jn);
         });
     } else {
         // R = A B: r = B a + b, t = t1 + A t2

@@ -214,8 +214,8 @@ solid_1d_kernel(const SolidArgs<T, AT> a, const int mt_max) {
 #pragma unroll
                 for (int c = 0; c < 3; c++) {
                     const C uc = U[c * 25 + k * 5 + jj], ur = U[c * 25 + ii * 5 + k];
-                    X[c].x += gx * uc.x; X[c].y += gx * uc.y;
-                    Y[c].x += ur.x * gy; Y[c].y += ur.y * gy;
+                    X[c] = cmac(X[c], uc, gx);
+                    Y[c] = cmac(Y[c], ur, gy);
                 }
             }
             const T alf = (T)al;
@@ -224,11 +224,11 @@ solid_1d_kernel(const SolidArgs<T, AT> a, const int mt_max) {
                 // ds, dz of the components, then A / s (on the axis dA / ds)
                 C S[3], o[3];
 #pragma unroll
-                for (int c = 0; c < 3; c++) S[c] = cadd(cscale(X[c], dze), cscale(Y[c], dzx));
+                for (int c = 0; c < 3; c++) S[c] = cmac(cscale(Y[c], dzx), X[c], dze);
                 eps[0] = S[0];
-                eps[4] = cadd(cadd(cscale(X[0], dse), cscale(Y[0], dsx)), S[2]);
-                eps[3] = cadd(cscale(X[1], dse), cscale(Y[1], dsx));
-                eps[2] = cadd(cscale(X[2], dse), cscale(Y[2], dsx));
+                eps[4] = cadd(cmac(cscale(Y[0], dsx), X[0], dse), S[2]);
+                eps[3] = cmac(cscale(Y[1], dsx), X[1], dse);
+                eps[2] = cmac(cscale(Y[2], dsx), X[2], dse);
                 eps[5] = S[1];
                 const bool lim = axial && ii == 0;
                 const C b0 = lim ? S[0] : U[q], b1 = lim ? S[1] : U[25 + q], b2 = lim ? S[2] : U[50 + q];
@@ -275,12 +275,12 @@ solid_1d_kernel(const SolidArgs<T, AT> a, const int mt_max) {
             A[0] = csub(cia(alf, sig[5]), sig[1]);
             A[1] = cadd(cia(alf, sig[1]), sig[5]);
             A[2] = cia(alf, sig[3]);
-            x[0] = cadd(cscale(sig[0], dze_i), cscale(sig[4], dse_i));
-            x[1] = cadd(cscale(sig[0], dzx_i), cscale(sig[4], dsx_i));
-            x[2] = cadd(cscale(sig[5], dze_i), cscale(sig[3], dse_i));
-            x[3] = cadd(cscale(sig[5], dzx_i), cscale(sig[3], dsx_i));
-            x[4] = cadd(cscale(sig[4], dze_i), cscale(sig[2], dse_i));
-            x[5] = cadd(cscale(sig[4], dzx_i), cscale(sig[2], dsx_i));
+            x[0] = cmac(cscale(sig[4], dse_i), sig[0], dze_i);
+            x[1] = cmac(cscale(sig[4], dsx_i), sig[0], dzx_i);
+            x[2] = cmac(cscale(sig[3], dse_i), sig[5], dze_i);
+            x[3] = cmac(cscale(sig[3], dsx_i), sig[5], dzx_i);
+            x[4] = cmac(cscale(sig[2], dse_i), sig[4], dze_i);
+            x[5] = cmac(cscale(sig[2], dsx_i), sig[4], dzx_i);
             if (axial && ii == 0) {
 #pragma unroll
                 for (int c = 0; c < 3; c++) {
@@ -307,8 +307,8 @@ solid_1d_kernel(const SolidArgs<T, AT> a, const int mt_max) {
 #pragma unroll
                 for (int c = 0; c < 3; c++) {
                     const C xv = xy[(2 * c) * 25 + k * 5 + jj], yv = xy[(2 * c + 1) * 25 + ii * 5 + k];
-                    f[c].x += gx * xv.x; f[c].y += gx * xv.y;
-                    f[c].x += yv.x * gt; f[c].y += yv.y * gt;
+                    f[c] = cmac(f[c], xv, gx);
+                    f[c] = cmac(f[c], yv, gt);
                 }
             }
 #pragma unroll

@@ -187,9 +187,9 @@ template <class V, class R>
 __device__ __forceinline__ void stress_iso(const V e[6], V s[6], R lam, R mu) {
     R mu2 = mu + mu;
     V sii = cscale(cadd(cadd(e[0], e[1]), e[2]), lam);
-    s[0] = cadd(sii, cscale(e[0], mu2));
-    s[1] = cadd(sii, cscale(e[1], mu2));
-    s[2] = cadd(sii, cscale(e[2], mu2));
+    s[0] = cmac(sii, e[0], mu2);
+    s[1] = cmac(sii, e[1], mu2);
+    s[2] = cmac(sii, e[2], mu2);
     s[3] = cscale(e[3], mu);
     s[4] = cscale(e[4], mu);
     s[5] = cscale(e[5], mu);
@@ -199,10 +199,10 @@ template <class V, class R>
 __device__ __forceinline__ void stress_tiso(const V e[6], V s[6], R A, R C, R F, R L, R Nn) {
     R mN2 = -(Nn + Nn);
     V t3 = cadd(e[0], e[1]);
-    V t4 = cadd(cscale(t3, A), cscale(e[2], F));
-    s[0] = cadd(t4, cscale(e[1], mN2));
-    s[1] = cadd(t4, cscale(e[0], mN2));
-    s[2] = cadd(cscale(t3, F), cscale(e[2], C));
+    V t4 = cmac(cscale(e[2], F), t3, A);
+    s[0] = cmac(t4, e[1], mN2);
+    s[1] = cmac(t4, e[0], mN2);
+    s[2] = cmac(cscale(e[2], C), t3, F);
     s[3] = cscale(e[3], L);
     s[4] = cscale(e[4], L);
     s[5] = cscale(e[5], Nn);
@@ -217,7 +217,7 @@ __device__ __forceinline__ void stress_aniso(const V e[6], V s[6], const R c[21]
     for (int i = 0; i < 6; i++) {
         V acc = cscale(e[0], c[idx[i][0]]);
 #pragma unroll
-        for (int j = 1; j < 6; j++) acc = cadd(acc, cscale(e[j], c[idx[i][j]]));
+        for (int j = 1; j < 6; j++) acc = cmac(acc, e[j], c[idx[i][j]]);
         s[i] = acc;
     }
 }
@@ -227,6 +227,7 @@ template <class T> struct re1 { T x; };
 template <class T> __device__ __forceinline__ re1<T> cadd(re1<T> a, re1<T> b) { return {a.x + b.x}; }
 template <class T> __device__ __forceinline__ re1<T> csub(re1<T> a, re1<T> b) { return {a.x - b.x}; }
 template <class T, class R> __device__ __forceinline__ re1<T> cscale(re1<T> a, R s) { return {a.x * (T)s}; }
+template <class T, class R> __device__ __forceinline__ re1<T> cmac(re1<T> acc, re1<T> a, R s) { return {acc.x + a.x * (T)s}; }
 
 template <int RHEO, class T, class V>
 __device__ __forceinline__ void elastic_at(const T *mod, int nslice, int slice, int q,
@@ -250,23 +251,23 @@ template <class V, class T>
 __device__ __forceinline__ void spz_to_rtz6(V e[6], T s1, T c1, T s2, T c2) {
     const T half = (T)0.5;
     V s02 = cadd(e[0], e[2]), d02 = csub(e[0], e[2]);
-    e[0] = cscale(csub(cadd(s02, cscale(d02, c2)), cscale(e[4], s2)), half);
+    e[0] = cscale(csub(cmac(s02, d02, c2), cscale(e[4], s2)), half);
     e[2] = csub(s02, e[0]);
-    e[4] = cadd(cscale(e[4], c2), cscale(d02, s2));
+    e[4] = cmac(cscale(e[4], c2), d02, s2);
     V t3 = e[3];
-    e[3] = cadd(cscale(t3, c1), cscale(e[5], s1));
+    e[3] = cmac(cscale(t3, c1), e[5], s1);
     e[5] = csub(cscale(e[5], c1), cscale(t3, s1));
 }
 template <class V, class T>
 __device__ __forceinline__ void rtz_to_spz6(V s[6], T s1, T c1, T s2, T c2) {
     const T half = (T)0.5;
     V s02 = cadd(s[0], s[2]), d02 = csub(s[0], s[2]);
-    s[0] = cadd(cscale(cadd(s02, cscale(d02, c2)), half), cscale(s[4], s2));
+    s[0] = cmac(cscale(cmac(s02, d02, c2), half), s[4], s2);
     s[2] = csub(s02, s[0]);
     s[4] = csub(cscale(s[4], c2), cscale(cscale(d02, s2), half));
     V t3 = s[3];
     s[3] = csub(cscale(t3, c1), cscale(s[5], s1));
-    s[5] = cadd(cscale(s[5], c1), cscale(t3, s1));
+    s[5] = cmac(cscale(s[5], c1), t3, s1);
 }
 
 // ----------------------------------------------------------- attenuation ---
@@ -483,27 +484,25 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
             const C *U = rBc + la * 75;
             C X[3], Y[3];
 #pragma unroll
-            for (int c = 0; c < 3; c++) {
-                C x = mk<T>(0, 0), y = mk<T>(0, 0);
+            for (int c = 0; c < 3; c++) { X[c] = mk<T>(0, 0); Y[c] = mk<T>(0, 0); }
 #pragma unroll
-                for (int k = 0; k < 5; k++) {
-                    const T gx = Gxi[k * 5 + ii];        // GT_xi(ii, k)
-                    const T gy = sGll[k * 5 + jj];       // G_GLL(k, jj)
-                    const C uc = U[c * 25 + k * 5 + jj];
-                    const C ur = U[c * 25 + ii * 5 + k];
-                    x.x += gx * uc.x; x.y += gx * uc.y;
-                    y.x += ur.x * gy; y.y += ur.y * gy;
+            for (int k = 0; k < 5; k++) {
+                const T gx = Gxi[k * 5 + ii];        // GT_xi(ii, k)
+                const T gy = sGll[k * 5 + jj];       // G_GLL(k, jj)
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    X[c] = cmac(X[c], U[c * 25 + k * 5 + jj], gx);
+                    Y[c] = cmac(Y[c], U[c * 25 + ii * 5 + k], gy);
                 }
-                X[c] = x; Y[c] = y;
             }
             const T ze = dzdeta[q], zx = dzdxii[q], se = dsdeta[q], sx = dsdxii[q];
             C eps[6], S[3];
 #pragma unroll
-            for (int c = 0; c < 3; c++) S[c] = cadd(cscale(X[c], ze), cscale(Y[c], zx));
+            for (int c = 0; c < 3; c++) S[c] = cmac(cscale(Y[c], zx), X[c], ze);
             eps[0] = S[0];
-            eps[4] = cadd(cadd(cscale(X[0], se), cscale(Y[0], sx)), S[2]);
-            eps[3] = cadd(cscale(X[1], se), cscale(Y[1], sx));
-            eps[2] = cadd(cscale(X[2], se), cscale(Y[2], sx));
+            eps[4] = cadd(cmac(cscale(Y[0], sx), X[0], se), S[2]);
+            eps[3] = cmac(cscale(Y[1], sx), X[1], se);
+            eps[2] = cmac(cscale(Y[2], sx), X[2], se);
             // lower-order terms A / s; on the axis (L'Hopital) dA / ds, the same combination of
             // the derivatives
             const T alf = (T)al;
@@ -589,14 +588,14 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
                     for (int i = lane; i < 25 * npb; i += TEAM) {
                         const int pb = (i / 5) % npb, n0 = 6 * ((i / (5 * npb)) * 5 + i % 5);
                         const int k0 = pb * KPc;
-                        T A[KPc][6], B[KPc][6];
+                        C AB[KPc][6];   // sums of Re cos and of Im sin, side by side
                         int j[KPc], kst[KPc];
 #pragma unroll
                         for (int kk = 0; kk < KPc; kk++) {
                             j[kk] = 0;
                             kst[kk] = k0 + kk < npair ? k0 + kk : 0;
 #pragma unroll
-                            for (int c = 0; c < 6; c++) { A[kk][c] = 0; B[kk][c] = 0; }
+                            for (int c = 0; c < 6; c++) AB[kk][c] = mk<T>(0, 0);
                         }
 #pragma unroll DFT_UNROLL
                         for (int al = 1; al < nu; al++) {
@@ -608,10 +607,7 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
                                 j[kk] = j[kk] >= nr ? j[kk] - nr : j[kk];
                                 const T2 w2 = tw2[j[kk]];
 #pragma unroll
-                                for (int c = 0; c < 6; c++) {
-                                    A[kk][c] += ev[c].x * w2.x;
-                                    B[kk][c] += ev[c].y * w2.y;
-                                }
+                                for (int c = 0; c < 6; c++) AB[kk][c] = cmacv(AB[kk][c], ev[c], w2);
                             }
                         }
                         C c0[6];
@@ -622,11 +618,11 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
                             if (k >= npair) break;
                             T x[6];
 #pragma unroll
-                            for (int c = 0; c < 6; c++) x[c] = c0[c].x + (T)2 * (A[kk][c] - B[kk][c]);
+                            for (int c = 0; c < 6; c++) x[c] = c0[c].x + (T)2 * (AB[kk][c].x - AB[kk][c].y);
                             st6r<T>(rBr + (size_t)k * 150 + n0, x);
                             if (k != 0 && 2 * k != nr) {
 #pragma unroll
-                                for (int c = 0; c < 6; c++) x[c] = c0[c].x + (T)2 * (A[kk][c] + B[kk][c]);
+                                for (int c = 0; c < 6; c++) x[c] = c0[c].x + (T)2 * (AB[kk][c].x + AB[kk][c].y);
                                 st6r<T>(rBr + (size_t)(nr - k) * 150 + n0, x);
                             }
                         }
@@ -636,14 +632,14 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
                 for (int i = lane; i < npb * qcnt; i += TEAM) {
                     const int pb = i / qcnt, qq = i - pb * qcnt, q = q0 + qq;
                     const int k0 = pb * KPc;
-                    T A[KPc][6], B[KPc][6];
+                    C AB[KPc][6];
                     int j[KPc], kst[KPc];
 #pragma unroll
                     for (int kk = 0; kk < KPc; kk++) {
                         j[kk] = 0;
                         kst[kk] = k0 + kk < npair ? k0 + kk : 0;
 #pragma unroll
-                        for (int d = 0; d < 6; d++) { A[kk][d] = 0; B[kk][d] = 0; }
+                        for (int d = 0; d < 6; d++) AB[kk][d] = mk<T>(0, 0);
                     }
                     for (int al = 1; al < nu; al++) {
                         C ev[6];
@@ -654,12 +650,8 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
                             j[kk] += kst[kk];
                             j[kk] = j[kk] >= nr ? j[kk] - nr : j[kk];
                             const T2 w2 = tw2[j[kk]];
-                            const T c = w2.x, sn = w2.y;
 #pragma unroll
-                            for (int d = 0; d < 6; d++) {
-                                A[kk][d] += ev[d].x * c;
-                                B[kk][d] += ev[d].y * sn;
-                            }
+                            for (int d = 0; d < 6; d++) AB[kk][d] = cmacv(AB[kk][d], ev[d], w2);
                         }
                     }
 #pragma unroll
@@ -670,8 +662,8 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
 #pragma unroll
                         for (int d = 0; d < 6; d++) {
                             const T c0 = rA[d * 25 + q].x;
-                            rBr[((size_t)k * 6 + d) * qcnt + qq] = c0 + (T)2 * (A[kk][d] - B[kk][d]);
-                            if (two) rBr[((size_t)(nr - k) * 6 + d) * qcnt + qq] = c0 + (T)2 * (A[kk][d] + B[kk][d]);
+                            rBr[((size_t)k * 6 + d) * qcnt + qq] = c0 + (T)2 * (AB[kk][d].x - AB[kk][d].y);
+                            if (two) rBr[((size_t)(nr - k) * 6 + d) * qcnt + qq] = c0 + (T)2 * (AB[kk][d].x + AB[kk][d].y);
                         }
                     }
                 }
@@ -857,39 +849,35 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
                     for (int i = lane; i < 25 * nab; i += TEAM) {
                         const int ab = (i / 5) % nab, n0 = 6 * ((i / (5 * nab)) * 5 + i % 5);
                         const int a0 = ab * ABc;
-                        T re[ABc][6], im[ABc][6];
+                        C ri[ABc][6];
                         int j[ABc], astep[ABc];
 #pragma unroll
                         for (int aa = 0; aa < ABc; aa++) {
                             j[aa] = 0;
                             astep[aa] = (a0 + aa) % nr;
 #pragma unroll
-                            for (int c = 0; c < 6; c++) { re[aa][c] = 0; im[aa][c] = 0; }
+                            for (int c = 0; c < 6; c++) ri[aa][c] = mk<T>(0, 0);
                         }
 #pragma unroll DFT_UNROLL
                         for (int k = 0; k <= nr / 2; k++) {
-                            T xs[6], xd[6];
+                            // (x_k + x_nr-k, x_nr-k - x_k) against (cos, sin)
+                            T xs[6];
+                            C p[6];
                             ld6r<T>(rBr + (size_t)k * 150 + n0, xs);
                             if (k != 0 && 2 * k != nr) {
                                 T x2[6];
                                 ld6r<T>(rBr + (size_t)(nr - k) * 150 + n0, x2);
 #pragma unroll
-                                for (int c = 0; c < 6; c++) {
-                                    xd[c] = xs[c] - x2[c];
-                                    xs[c] += x2[c];
-                                }
+                                for (int c = 0; c < 6; c++) p[c] = mk<T>(xs[c] + x2[c], x2[c] - xs[c]);
                             } else {
 #pragma unroll
-                                for (int c = 0; c < 6; c++) xd[c] = xs[c];
+                                for (int c = 0; c < 6; c++) p[c] = mk<T>(xs[c], -xs[c]);
                             }
 #pragma unroll
                             for (int aa = 0; aa < ABc; aa++) {
                                 const T2 w2 = tw2[j[aa]];
 #pragma unroll
-                                for (int c = 0; c < 6; c++) {
-                                    re[aa][c] += xs[c] * w2.x;
-                                    im[aa][c] -= xd[c] * w2.y;
-                                }
+                                for (int c = 0; c < 6; c++) ri[aa][c] = cmacv(ri[aa][c], p[c], w2);
                                 j[aa] += astep[aa];
                                 j[aa] = j[aa] >= nr ? j[aa] - nr : j[aa];
                             }
@@ -903,7 +891,7 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
                             const bool noim = al == 0 || nyq;
                             C sg[6];
 #pragma unroll
-                            for (int c = 0; c < 6; c++) sg[c] = mk<T>(re[aa][c] * sr, noim ? (T)0 : im[aa][c] * inv_nr);
+                            for (int c = 0; c < 6; c++) sg[c] = mk<T>(ri[aa][c].x * sr, noim ? (T)0 : ri[aa][c].y * inv_nr);
                             st6c<T>(rA + al * 150 + n0, sg);
                         }
                     }
@@ -984,12 +972,12 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
             A[0] = csub(cia(alf, s[5]), s[1]);
             A[1] = cadd(cia(alf, s[1]), s[5]);
             A[2] = cia(alf, s[3]);
-            x[0] = cadd(cscale(s[0], ze), cscale(s[4], se));
-            x[1] = cadd(cscale(s[0], zx), cscale(s[4], sx));
-            x[2] = cadd(cscale(s[5], ze), cscale(s[3], se));
-            x[3] = cadd(cscale(s[5], zx), cscale(s[3], sx));
-            x[4] = cadd(cscale(s[4], ze), cscale(s[2], se));
-            x[5] = cadd(cscale(s[4], zx), cscale(s[2], sx));
+            x[0] = cmac(cscale(s[4], se), s[0], ze);
+            x[1] = cmac(cscale(s[4], sx), s[0], zx);
+            x[2] = cmac(cscale(s[3], se), s[5], ze);
+            x[3] = cmac(cscale(s[3], sx), s[5], zx);
+            x[4] = cmac(cscale(s[2], se), s[4], ze);
+            x[5] = cmac(cscale(s[2], sx), s[4], zx);
             if (axial && q < 5) {
 #pragma unroll
                 for (int c = 0; c < 3; c++) {
@@ -1022,8 +1010,8 @@ solid_stiffness_kernel(const SolidArgs<T, AT> a, const int nr_max, const int qc_
                 for (int c = 0; c < 3; c++) {
                     const C xv = xy[(2 * c) * 25 + k * 5 + jj];
                     const C yv = xy[(2 * c + 1) * 25 + ii * 5 + k];
-                    f[c].x += gx * xv.x; f[c].y += gx * xv.y;
-                    f[c].x += yv.x * gt; f[c].y += yv.y * gt;
+                    f[c] = cmac(f[c], xv, gx);
+                    f[c] = cmac(f[c], yv, gt);
                 }
             }
             if constexpr (sizeof(T) == 4) {

@@ -131,3 +131,40 @@ def test_cg4_slices_match_oracle(built, nr):
             s.set_field(u, "displ")
             s.run(4)
             assert np.linalg.norm(s.get_field("displ") - d) <= TOL["mixed"] * np.linalg.norm(d)
+
+
+@pytest.mark.parametrize("pieces", [[64], [1, 7, 8, 48], [15, 16, 17, 16], [33, 31]])
+def test_step_graphs_of_one_and_several_steps(built, pieces):
+    """Runs of any length replay graphs of eight steps and of one: the same steps, records and
+    source times as launch by launch."""
+    m = meshgen.cartesian_model(nx=7, nz=5, nr=5, nstations=4, record_interval=3)
+    with Solver(m, "fp64") as s:
+        s.run(64, graph=False)
+        ref, seis = s.get_field("displ"), s.seismograms()
+    with Solver(m, "fp64") as s:
+        for n in pieces:
+            s.run(n)
+        assert s.step == 64
+        d, g = s.get_field("displ"), s.seismograms()
+    assert np.linalg.norm(d - ref) <= 1e-12 * np.linalg.norm(ref)
+    assert g.shape == seis.shape and np.linalg.norm(g - seis) <= 1e-12 * np.linalg.norm(seis)
+
+
+def test_more_wavefields_than_one_grid_axis(built):
+    """A wavefield beyond the 32768 rows of the point update's second grid axis is updated too."""
+    m = meshgen.microbench_model(n_elem=1, nr_choices=[1], is3d=False, rheology="iso", attenuation=None, seed=3)
+    u = meshgen.random_displacement(m, seed=4)
+    with Solver(m, "fp32") as s:
+        s.set_field(u, "displ")
+        s.run(3)
+        one = s.get_field("displ")
+    m.nwave = 32770
+    full = np.zeros((m.nwave, u.size), np.complex128)
+    full[0] = full[-1] = u
+    with Solver(m, "fp32") as s:
+        s.set_field(full.ravel(), "displ")
+        s.run(3)
+        got = s.get_field("displ").reshape(m.nwave, -1)
+    assert not np.any(got[1:-1])
+    for w in (0, -1):
+        assert np.linalg.norm(got[w] - one) <= 1e-6 * np.linalg.norm(one)

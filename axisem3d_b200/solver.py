@@ -11,7 +11,7 @@ NewmarkTimeScheme::solve (SOLVER/src/core/time/NewmarkTimeScheme.cpp:41-108):
     apply_bc_after_assembly()  Domain::applyBC_AfterAssemblingStiff
     stiff_to_accel()           Domain::computeStiffToAccel
     newmark_update()           NewmarkTimeScheme::update on all points
-    run(nsteps)                the whole loop body, one CUDA graph per step
+    run(nsteps)                the whole loop body as CUDA graphs of one or several steps
 
 Errors raise ``RuntimeError`` with the engine's "Class::method || message"
 text, as the reference throws std::runtime_error.

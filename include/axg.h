@@ -393,7 +393,8 @@ int  axg_newmark_update(axg_solver *h);
 /* station recording of the displacement at step tstep */
 int  axg_record_stations(axg_solver *h, int32_t tstep);
 /* nsteps full Newmark steps starting at the handle's step counter
-   (NewmarkTimeScheme::solve loop body); use_graph = 1 replays one CUDA graph per step */
+   (NewmarkTimeScheme::solve loop body); use_graph = 1 replays CUDA graphs of
+   one or several steps */
 int  axg_run(axg_solver *h, int32_t nsteps, int32_t use_graph);
 /* step counter of the next step */
 int  axg_current_step(const axg_solver *h, int32_t *tstep);

@@ -1268,7 +1268,13 @@ private:
             std::vector<T> xpool;
             std::vector<int64_t> xoff;
             std::vector<uint8_t> x3d;
-            const std::vector<int> &ids = kv.second;
+            std::vector<int> &ids = kv.second;
+            // The largest elements first where a bucket is about one wave of blocks, so that what is
+            // left over for a second one is the cheapest: 154 elements of nr 120 .. 250 110 -> 101 us.
+            // Larger buckets keep the mesh's order, in which neighbours share the lines of their
+            // points (sorted up to 8 waves: 1 % slower, up to 64: 2 - 3 %).
+            if (!cfg_.plain && b->is3d && (int)ids.size() < 2 * prop_.multiProcessorCount)
+                std::stable_sort(ids.begin(), ids.end(), [&](int x, int y) { return h.nr[x] > h.nr[y]; });
             b->n = (int)ids.size();
             b->nr_max = 1;
             std::vector<int> nr(b->n), pts((size_t)b->n * 25);

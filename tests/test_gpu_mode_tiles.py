@@ -168,3 +168,16 @@ def test_more_wavefields_than_one_grid_axis(built):
     assert not np.any(got[1:-1])
     for w in (0, -1):
         assert np.linalg.norm(got[w] - one) <= 1e-6 * np.linalg.norm(one)
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_small_buckets_largest_elements_first(built, precision):
+    """A bucket of about one wave of blocks runs in the order of falling nr: state, moduli and
+    offsets follow their elements, step after step."""
+    m = meshgen.microbench_model(n_elem=40, nr_min=26, nr_max=64, seed=17)
+    u = meshgen.random_displacement(m, seed=8)
+    f, d = _oracle_steps(m, u, 4)
+    with Solver(m, precision) as s:
+        s.set_field(u, "displ")
+        s.run(4)
+        assert np.linalg.norm(s.get_field("displ") - d) <= TOL[precision] * np.linalg.norm(d)

@@ -25,13 +25,18 @@
 
 namespace axg {
 
+// A failed call throws and takes the runtime's record of its error with it: the check after a
+// kernel launch reads that record, and would report it for the next launch of any handle of the
+// thread.
 #define AXG_CUDA(call)                                                                       \
     do {                                                                                     \
         cudaError_t e_ = (call);                                                             \
-        if (e_ != cudaSuccess)                                                               \
+        if (e_ != cudaSuccess) {                                                             \
+            cudaGetLastError();                                                              \
             throw Error(e_ == cudaErrorMemoryAllocation ? AXG_E_NOMEM : AXG_E_CUDA,          \
                         std::string("Engine::" ) + __func__ + " || " + #call + " || " +      \
                             cudaGetErrorString(e_));                                         \
+        }                                                                                    \
     } while (0)
 
 // owning device buffer
@@ -2445,7 +2450,7 @@ private:
 
     void post_launch() {
         launches_++;
-        cudaError_t e = cudaPeekAtLastError();
+        cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess)
             throw Error(AXG_E_CUDA, std::string("Engine::launch || ") + cudaGetErrorString(e));
     }
@@ -2466,6 +2471,7 @@ private:
             for (int i = 0; i < steps; i++) launch_step();
         } catch (...) {
             cudaStreamEndCapture(stream_, &g);
+            cudaGetLastError();
             throw;
         }
         AXG_CUDA(cudaStreamEndCapture(stream_, &g));

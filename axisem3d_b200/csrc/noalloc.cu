@@ -32,9 +32,11 @@ void *noalloc_scratch(int device) {
             e = cudaGetSymbolAddress(&p, axg_noalloc_scratch);
             cudaSetDevice(prev);
         }
-        if (e != cudaSuccess || !p)
+        if (e != cudaSuccess || !p) {
+            cudaGetLastError();
             throw Error(AXG_E_CUDA, std::string("axg_compute_stiffness_noalloc || cudaGetSymbolAddress: ") +
                                         cudaGetErrorString(e));
+        }
         addr[device] = p;
     }
     return addr[device];

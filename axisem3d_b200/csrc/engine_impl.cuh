@@ -1538,10 +1538,12 @@ private:
         b.grid = (b.n + tpc - 1) / tpc;
     }
 
-    // The project's autotuner: for every solid bucket, time each feasible team size
-    // (threads per element) on the bucket's own elements and keep the fastest. The
-    // fields are zero at this point, so the trial launches change no result; the
-    // attenuation state and the stiffness are cleared afterwards all the same.
+    // The project's autotuner: for every solid bucket, time the default and each feasible team
+    // size (threads per element) on the bucket's own elements and keep the fastest. The default
+    // is a candidate of its own: 1-D buckets have tiles that no team size gives, and 3-D elements
+    // too large for two blocks per SM a 512-thread block (FP64 elastic elements of nr = 75: 251 us
+    // per step, 396 with 256 threads). The fields are zero at this point, so the trial launches
+    // change no result; the attenuation state and the stiffness are cleared afterwards all the same.
     void autotune() {
         cudaEvent_t t0, t1;
         AXG_CUDA(cudaEventCreate(&t0));
@@ -1549,10 +1551,11 @@ private:
         for (auto &bp : sb_) {
             SolidBucket &b = *bp;
             float best = 1e30f;
-            int best_team = b.kernel1d ? 0 : b.team;
+            int best_team = 0, default_threads = 0;
             for (int team : {0, 32, 64, 128, 256}) {
-                if (team == 0 && !b.kernel1d) continue;   // 1-D buckets: the default tiles as well
+                if (team && team == default_threads && !b.kernel1d) continue;   // the default, timed already
                 configure_bucket(b, team);
+                if (team == 0) default_threads = b.team;
                 float ms = 0;
                 for (int rep = 0; rep < 3; rep++) {
                     AXG_CUDA(cudaEventRecord(t0, stream_));
@@ -1566,7 +1569,6 @@ private:
                 if (ms < best) { best = ms; best_team = team; }
             }
             configure_bucket(b, best_team);
-            tuned_.push_back({b.cls, b.team, best / 2});
         }
         cudaEventDestroy(t0);
         cudaEventDestroy(t1);
@@ -2499,8 +2501,6 @@ private:
     cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;
     cudaGraphExec_t graph_exec_ = nullptr, graph_multi_ = nullptr;   // one step, kGraphSteps steps
     int team_override_[kNrClasses];
-    struct Tuned { int cls, team; float ms; };
-    std::vector<Tuned> tuned_;
     // differentiation
     DBuf<CD> ck_displ_, ck_veloc_;
     DBuf<C> ck_accel_;

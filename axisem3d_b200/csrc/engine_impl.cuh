@@ -308,21 +308,25 @@ public:
                 time_n_ += 1;
             }
         } else if (graph && !cfg_.plain) {
-            // several steps in one graph while there are enough of them: a graph's start and end
-            // cost a small mesh's step about as much as one of its kernels
-            int i = 0;
-            if (nsteps >= 2 * kGraphSteps) {
-                if (!graph_multi_) capture(graph_multi_, kGraphSteps);
-                for (; i + kGraphSteps <= nsteps; i += kGraphSteps) {
-                    AXG_CUDA(cudaGraphLaunch(graph_multi_, stream_));
-                    launches_ += kernels_per_step_ * kGraphSteps;
+            int left = nsteps;
+            auto replay = [&](StepGraph &g, int steps) {
+                refresh(g, steps);
+                AXG_CUDA(cudaGraphLaunch(g.exec, stream_));
+                launches_ += kernels_per_step_ * steps;
+                left -= steps;
+            };
+            // Several steps in one graph where a handle runs enough of them: a graph's start and end
+            // cost a small mesh's step about as much as one of its kernels. Building it is host time,
+            // so the steps ahead of it are queued first and the GPU runs them meanwhile.
+            if (nsteps >= kGraphSteps) asked_ += nsteps;
+            if (asked_ >= kManySteps && nsteps >= kGraphSteps) {
+                if (!many_.exec) {
+                    for (int k = 0; k < kLeadSteps && left > 0; k++) replay(one_, 1);
+                    refresh(many_, kGraphSteps);
                 }
+                while (left >= kGraphSteps) replay(many_, kGraphSteps);
             }
-            if (i < nsteps && !graph_exec_) capture(graph_exec_, 1);
-            for (; i < nsteps; i++) {
-                AXG_CUDA(cudaGraphLaunch(graph_exec_, stream_));
-                launches_ += kernels_per_step_;
-            }
+            while (left > 0) replay(one_, 1);
         } else {
             for (int i = 0; i < nsteps; i++) launch_step();
         }
@@ -630,14 +634,14 @@ public:
             dev_step_ = -1;
             // recompute the segment, keeping u_n and a_n (the forward step's graph, which reads
             // the step from the device counter set above)
-            if (!cfg_.plain && !graph_exec_) capture(graph_exec_, 1);
+            if (!cfg_.plain) refresh(one_, 1);
             for (int i = 0; i < len; i++) {
                 AXG_CUDA(cudaMemcpyAsync(seg_u.p + nf * i, sp_.displ.p, nf * sizeof(C),
                                          cudaMemcpyDeviceToDevice, stream_));
                 if (cfg_.plain) {
                     launch_step();
                 } else {
-                    AXG_CUDA(cudaGraphLaunch(graph_exec_, stream_));
+                    AXG_CUDA(cudaGraphLaunch(one_.exec, stream_));
                     launches_ += kernels_per_step_;
                 }
                 AXG_CUDA(cudaMemcpyAsync(seg_a.p + nf * i, sp_.accel.p, nf * sizeof(C),
@@ -1986,16 +1990,16 @@ private:
 
     // STF table and seismogram buffer large enough for steps [0, nsteps)
     void ensure_capacity(int nsteps) {
-        bool changed = false;
         if ((ms_n_ || fs_n_ || ps_n_) && nsteps > stf_valid_) {
             int cap = std::max(nsteps, 2 * stf_cap_);
+            one_.stale = many_.stale = true;
             fill_stf(cap, nsteps);
-            changed = true;
         }
         if (st_n_) {
             int need_rec = (nsteps + st_interval_ - 1) / st_interval_;
             if (need_rec > seis_cap_) {
                 int cap = std::max(need_rec, 2 * seis_cap_);
+                one_.stale = many_.stale = true;
                 DBuf<double> nb;
                 nb.alloc((size_t)cap * nwave_ * st_n_ * 3);
                 nb.zero(stream_);
@@ -2016,10 +2020,8 @@ private:
                     std::swap(seis_grad_.p, ng.p); std::swap(seis_grad_.n, ng.n);
                 }
                 seis_cap_ = cap;
-                changed = true;
             }
         }
-        if (changed) drop_graphs();
     }
     static T src_stf(const HostSources &h, int i, double t) {
         auto it = h.table.find(i);
@@ -2457,30 +2459,61 @@ private:
             throw Error(AXG_E_CUDA, std::string("Engine::launch || ") + cudaGetErrorString(e));
     }
 
-    static constexpr int kGraphSteps = 8;
+    // Captured steps. The graph of eight of them costs a small mesh 0.7 (40 x 40 box) to 1.4 ms (1-D
+    // globe, 9 launches per step) to instantiate and about as much to destroy, and saves 3.5 and 10 us
+    // a step: it is made once a handle has been asked for kManySteps steps in runs that can use it,
+    // behind kLeadSteps queued ones. Made in every run of 16 steps or more, and again at each growth
+    // of the tables, it cost the first three runs of 20 steps 1.1, 1.9 and 1.9 ms on the box and 2.5,
+    // 4.1 and 4.4 on the globe; this way 0.6, 0.4, 0.4 and 1.6, 1.1, 1.5, and 100 steps of a handle
+    // in use are what they were (1.35 and 4.60 ms).
+    static constexpr int kGraphSteps = 8, kManySteps = 256, kLeadSteps = 64;
+    struct StepGraph {
+        cudaGraphExec_t exec = nullptr;
+        bool stale = true;    // a table of the step has moved since the capture
+    };
     void drop_graphs() {
-        for (cudaGraphExec_t *e : {&graph_exec_, &graph_multi_}) {
-            if (*e) cudaGraphExecDestroy(*e);
-            *e = nullptr;
+        for (StepGraph *g : {&one_, &many_}) {
+            if (g->exec) cudaGraphExecDestroy(g->exec);
+            *g = StepGraph();
         }
+        asked_ = 0;
     }
-    // `steps` time steps, which read and advance the device step counter, as one graph
-    void capture(cudaGraphExec_t &exec, int steps) {
+    // `steps` time steps, which read and advance the device step counter, as one graph, up to date:
+    // tables that have moved change the parameters of its launches and not their order, which an
+    // instantiated graph takes over in a few microseconds a launch
+    void refresh(StepGraph &s, int steps) {
+        if (s.exec && !s.stale) return;
+        cudaGraph_t g = capture(steps);
+        cudaError_t e = cudaErrorGraphExecUpdateFailure;
+        cudaGraphExecUpdateResultInfo info;
+        if (s.exec) e = cudaGraphExecUpdate(s.exec, g, &info);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            if (s.exec) cudaGraphExecDestroy(s.exec);
+            s.exec = nullptr;
+            e = cudaGraphInstantiate(&s.exec, g, 0);
+            if (e != cudaSuccess) s.exec = nullptr;
+        }
+        cudaGraphDestroy(g);
+        AXG_CUDA(e);
+        s.stale = false;
+    }
+    cudaGraph_t capture(int steps) {
         cudaGraph_t g;
-        int64_t before = launches_;
+        const int64_t before = launches_;
         AXG_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
         try {
             for (int i = 0; i < steps; i++) launch_step();
         } catch (...) {
             cudaStreamEndCapture(stream_, &g);
             cudaGetLastError();
+            launches_ = before;
             throw;
         }
         AXG_CUDA(cudaStreamEndCapture(stream_, &g));
         kernels_per_step_ = (launches_ - before) / steps;
         launches_ = before;
-        AXG_CUDA(cudaGraphInstantiate(&exec, g, 0));
-        cudaGraphDestroy(g);
+        return g;
     }
 
     // ---------------------------------------------------------------- data ---
@@ -2499,7 +2532,8 @@ private:
     double time_ms_ = 0;
     int64_t time_n_ = 0;
     cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;
-    cudaGraphExec_t graph_exec_ = nullptr, graph_multi_ = nullptr;   // one step, kGraphSteps steps
+    StepGraph one_, many_;                // of one step, of kGraphSteps steps
+    int64_t asked_ = 0;                   // steps of the runs long enough for many_, since the graphs were dropped
     int team_override_[kNrClasses];
     // differentiation
     DBuf<CD> ck_displ_, ck_veloc_;

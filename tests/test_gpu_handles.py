@@ -1,5 +1,7 @@
 """What handles choose for themselves, and what those of one process share or keep between calls: the
-autotuner's team sizes, the runtime's record of an error."""
+autotuner's team sizes, the captured steps, the runtime's record of an error."""
+import time
+
 import numpy as np
 import pytest
 
@@ -62,3 +64,38 @@ def test_autotuner_keeps_the_large_blocks(built):
         assert _block_threads(s, u) == [256]
     with Solver(m, "fp64", autotune=True) as s:
         assert _block_threads(s, u) == [512]
+
+
+@pytest.mark.parametrize("pieces", [[300], [20] * 15, [100, 100, 100], [8, 255, 1, 7, 9, 20], [250, 8, 42]])
+def test_graph_of_several_steps_behind_single_ones(built, pieces):
+    """The graph of eight steps is made once a handle has been asked for 256 steps, behind queued
+    single ones; source and record tables grow between the runs and both graphs follow them."""
+    m = meshgen.cartesian_model(nx=5, nz=4, nr=5, nstations=3, record_interval=7)
+    with Solver(m, "fp64") as s:
+        s.run(300, graph=False)
+        ref, seis = s.get_field("displ"), s.seismograms()
+    with Solver(m, "fp64") as s:
+        for n in pieces:
+            s.run(n)
+        assert s.step == 300
+        d, g = s.get_field("displ"), s.seismograms()
+    # the order of the atomic sums, over 300 steps
+    assert np.linalg.norm(d - ref) <= 1e-11 * np.linalg.norm(ref)
+    assert g.shape == seis.shape and np.linalg.norm(g - seis) <= 1e-11 * np.linalg.norm(seis)
+
+
+def test_short_runs_do_not_pay_for_graphs(built):
+    """Runs of 20 steps of a new handle, the tables growing under them, take no longer than twice
+    their launches one by one (three to four times with graphs of eight steps made for each)."""
+    m = meshgen.cartesian_model(nx=40, nz=40, nr=5, nstations=20)
+    best = {}
+    for graph in (False, True) * 4:
+        with Solver(m, "fp32") as s:
+            s.run(20, graph=graph)
+            s.synchronize()
+            t = time.perf_counter()
+            for _ in range(2):
+                s.run(20, graph=graph)
+                s.synchronize()
+            best[graph] = min(best.get(graph, 1.0), time.perf_counter() - t)
+    assert best[True] <= 2 * best[False], best

@@ -1993,6 +1993,7 @@ private:
         if ((ms_n_ || fs_n_ || ps_n_) && nsteps > stf_valid_) {
             int cap = std::max(nsteps, 2 * stf_cap_);
             one_.stale = many_.stale = true;
+            AXG_CUDA(cudaStreamSynchronize(stream_));   // queued steps read the table that is given back
             fill_stf(cap, nsteps);
         }
         if (st_n_) {

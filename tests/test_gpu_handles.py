@@ -1,5 +1,6 @@
 """What handles choose for themselves, and what those of one process share or keep between calls: the
-autotuner's team sizes, the captured steps, the runtime's record of an error."""
+autotuner's team sizes, the captured steps, the step counter and the tables of a hook loop, the
+runtime's record of an error."""
 import time
 
 import numpy as np
@@ -99,3 +100,68 @@ def test_short_runs_do_not_pay_for_graphs(built):
                 s.synchronize()
             best[graph] = min(best.get(graph, 1.0), time.perf_counter() - t)
     assert best[True] <= 2 * best[False], best
+
+
+def _hooks(s, t):
+    s.apply_sources(t)
+    s.compute_stiffness()
+    s.apply_bc_before_assembly()
+    s.record_stations(t)
+    s.apply_bc_after_assembly()
+    s.stiff_to_accel()
+    s.newmark_update()
+
+
+def test_hooks_queue_steps_while_the_tables_grow(built):
+    """A hook loop that nothing waits in, from an empty source table: each growth gives the old
+    table back only when the queued steps have read it."""
+    m = meshgen.cartesian_model(nx=12, nz=9, nr=5, nstations=3)
+    with Solver(m, "fp64") as s:
+        s.run(200)
+        ref = s.get_field("displ")
+    with Solver(m, "fp64") as s:
+        for t in range(200):
+            _hooks(s, t)
+        d = s.get_field("displ")
+    assert np.linalg.norm(d - ref) <= 1e-11 * np.linalg.norm(ref)
+
+
+def test_hooks_runs_and_streams_in_turn(built):
+    """The device's step counter is set only when it does not hold the step already: hooks before and
+    after a run, a repeated step and a change of stream each record and shake the step they are given."""
+    import torch
+    n, interval = 24, 2
+    m = meshgen.cartesian_model(nx=6, nz=5, nr=5, nstations=4, record_interval=interval)
+    u0, other = (meshgen.random_displacement(m, seed=k) * 1e-3 for k in (9, 10))
+    with Solver(m, "fp64") as s:
+        s.set_field(u0, "displ")
+        s.run(n)
+        ref, seis = s.get_field("displ"), s.seismograms()
+    stream = torch.cuda.Stream()
+    with Solver(m, "fp64") as s:
+        # records of another wavefield in every slot, so that one left out shows
+        s.set_field(other, "displ")
+        s.run(n)
+        assert np.linalg.norm(s.seismograms() - seis) > 0.1 * np.linalg.norm(seis)
+        zero = np.zeros_like(u0)
+        for name, v in (("displ", u0), ("veloc", zero), ("accel", zero), ("stiff", zero)):
+            s.set_field(v, name)
+        for t in range(n):
+            _hooks(s, t)
+            if t in (5, 6, 15):
+                # a run elsewhere in time, then the fields as they were
+                keep = {k: s.get_field(k) for k in ("displ", "veloc", "accel", "stiff")}
+                k0 = s.step
+                s.run(3 if t == 15 else t)
+                assert s.step > k0
+                for k, v in keep.items():
+                    s.set_field(v, k)
+            if t == 10:
+                s.synchronize()
+                s.set_stream(stream.cuda_stream)
+            if t == 18:
+                s.synchronize()
+                s.set_stream(None)
+        d, g = s.get_field("displ"), s.seismograms()
+    assert np.linalg.norm(d - ref) <= 1e-12 * np.linalg.norm(ref)
+    assert np.linalg.norm(g[:seis.shape[0]] - seis) <= 1e-12 * np.linalg.norm(seis)

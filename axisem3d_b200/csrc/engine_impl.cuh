@@ -39,6 +39,13 @@ namespace axg {
         }                                                                                    \
     } while (0)
 
+// Host to device, there on return. A copy from pageable memory may return when it is staged, and no
+// handle's stream (nor a caller's non-blocking one) waits for the legacy stream that it runs on.
+inline void copy_in(void *dst, const void *src, size_t bytes) {
+    AXG_CUDA(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice));
+    AXG_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+}
+
 // owning device buffer
 template <class X>
 struct DBuf {
@@ -58,7 +65,7 @@ struct DBuf {
     void zero(cudaStream_t s) { if (n) AXG_CUDA(cudaMemsetAsync(p, 0, n * sizeof(X), s)); }
     void upload(const std::vector<X> &h) {
         alloc(h.size());
-        if (n) AXG_CUDA(cudaMemcpy(p, h.data(), n * sizeof(X), cudaMemcpyHostToDevice));
+        if (n) copy_in(p, h.data(), n * sizeof(X));
     }
 };
 
@@ -368,12 +375,11 @@ public:
         if (which == AXG_FIELD_DISPL || which == AXG_FIELD_VELOC) {
             std::vector<CD> h(n);
             for (size_t i = 0; i < n; i++) h[i] = mk<D>((D)in[2 * i], (D)in[2 * i + 1]);
-            AXG_CUDA(cudaMemcpy(which == AXG_FIELD_DISPL ? P.displ.p : P.veloc.p, h.data(),
-                                n * sizeof(CD), cudaMemcpyHostToDevice));
+            copy_in(which == AXG_FIELD_DISPL ? P.displ.p : P.veloc.p, h.data(), n * sizeof(CD));
             if (which == AXG_FIELD_DISPL && P.displ_elem.p) {
                 std::vector<C> hf(n);
                 for (size_t i = 0; i < n; i++) hf[i] = mk<T>((T)h[i].x, (T)h[i].y);
-                AXG_CUDA(cudaMemcpy(P.displ_elem.p, hf.data(), n * sizeof(C), cudaMemcpyHostToDevice));
+                copy_in(P.displ_elem.p, hf.data(), n * sizeof(C));
             }
             if (COMP) {
                 if (which == AXG_FIELD_DISPL) P.cd.zero(stream_); else P.cv.zero(stream_);
@@ -381,8 +387,7 @@ public:
         } else {
             std::vector<C> h(n);
             for (size_t i = 0; i < n; i++) h[i] = mk<T>((T)in[2 * i], (T)in[2 * i + 1]);
-            AXG_CUDA(cudaMemcpy(which == AXG_FIELD_STIFF ? P.stiff.p : P.accel.p, h.data(),
-                                n * sizeof(C), cudaMemcpyHostToDevice));
+            copy_in(which == AXG_FIELD_STIFF ? P.stiff.p : P.accel.p, h.data(), n * sizeof(C));
         }
         AXG_CUDA(cudaStreamSynchronize(stream_));
     }

@@ -134,7 +134,6 @@ class Engine final : public EngineBase {
         int n = 0, ndim = 3, total = 0, n3d = 0, nr_max = 1;
         std::vector<int> h_off, h_nu, h_nr;
         std::vector<uint8_t> h_flags;
-        std::vector<T> h_inv1;
         DBuf<uint8_t> mode_flags;
         DBuf<T> mode_inv;
         DBuf<int> off, nu, nr, mode_pt, pt3d;
@@ -222,8 +221,8 @@ public:
         build_points(m.sp, sp_, true);
         build_points(m.fp, fp_, false);
         build_ocean(m);
-        upload_mode_tables(sp_, true);
-        upload_mode_tables(fp_, false);
+        build_mode_tables(sp_, true);
+        build_mode_tables(fp_, false);
         // twiddles for every nr in use (3-D elements and Mass3D points)
         std::vector<int> nrs;
         int nrmax = 1;
@@ -485,6 +484,7 @@ public:
         er_out_.alloc((size_t)ring * nwave_ * (size_t)std::max<int64_t>(words, 1));
         er_out_.zero(stream_);
         if (n) upload_elem_tables(grad);
+        build_side_streams();
         AXG_CUDA(cudaStreamSynchronize(stream_));
         drop_graphs();
     }
@@ -1182,7 +1182,6 @@ private:
         P.mode_pt.upload(mode_pt); P.pt3d.upload(pt3d);
         P.flags.upload(flags); P.inv1.upload(inv1);
         P.h_flags = flags;
-        P.h_inv1 = inv1;
         if (inv3.empty()) inv3.push_back((T)0);
         P.inv3.upload(inv3); P.im_off.upload(im_off);
         size_t nf = (size_t)P.total * P.ndim * nwave_;
@@ -1194,28 +1193,13 @@ private:
         if (COMP) { P.cd.alloc(nf); P.cd.zero(stream_); P.cv.alloc(nf); P.cv.zero(stream_); }
     }
     // per mode: what the point update does to it (MODE_*) and its point's 1 / M
-    void upload_mode_tables(PointDev &P, bool solid) {
-        std::vector<uint8_t> mf;
-        std::vector<T> mi;
-        mf.reserve(P.total); mi.reserve(P.total);
-        for (int p = 0; p < P.n; p++) {
-            const uint8_t fl = P.h_flags[p];
-            const int nr = P.h_nr[p], nu = P.h_nu[p];
-            for (int al = 0; al < nu; al++) {
-                uint8_t b = 0;
-                if (fl & (PT_MASS3D | PT_OCEAN)) b |= MODE_SKIP;
-                if (fl & PT_AXIAL) {
-                    if (solid) b |= al == 0 ? MODE_AXIS0 : al == 1 ? MODE_AXIS1 : MODE_ZERO;
-                    else if (al >= 1) b |= MODE_ZERO;
-                }
-                if (!solid && (fl & PT_SURFACE)) b |= MODE_ZERO;
-                if ((nr & 1) == 0 && al == nu - 1) b |= MODE_NYQUIST;
-                mf.push_back(b);
-                mi.push_back(P.h_inv1[p]);
-            }
-        }
-        P.mode_flags.upload(mf);
-        P.mode_inv.upload(mi);
+    void build_mode_tables(PointDev &P, bool solid) {
+        P.mode_flags.alloc(P.total);
+        P.mode_inv.alloc(P.total);
+        if (!P.total) return;
+        mode_table_kernel<T><<<(P.total + 255) / 256, 256, 0, stream_>>>(P.total, solid, P.mode_pt.p, P.off.p, P.nr.p,
+                                                                        P.flags.p, P.inv1.p, P.mode_flags.p, P.mode_inv.p);
+        AXG_CUDA(cudaGetLastError());
     }
     // displacement as seen by the elements
     const C *elem_displ(const PointDev &P) const {
@@ -1378,9 +1362,12 @@ private:
             b->bytes = bytes;
             b->flops = flops;
             b->nr.upload(nr); b->pts.upload(pts); b->axial.upload(ax);
-            std::vector<int2> tab((size_t)b->n * 25);
-            for (size_t i = 0; i < tab.size(); i++) tab[i] = make_int2(sp_.h_off[pts[i]], sp_.h_nu[pts[i]]);
-            b->tab.upload(tab);
+            if (!b->prt) {
+                b->tab.alloc((size_t)b->n * 25);
+                offset_table_kernel<T><<<(b->n * 25 + 255) / 256, 256, 0, stream_>>>(b->n * 25, b->pts.p, sp_.off.p,
+                                                                                    sp_.nu.p, b->tab.p);
+                AXG_CUDA(cudaGetLastError());
+            }
             b->geom.upload(geom);
             if (trig.empty()) trig.push_back((T)0);
             b->trig.upload(trig);
@@ -2116,14 +2103,16 @@ private:
         post_launch();
     }
 
-    // the side streams of run_branches, as many as the step has branches beyond the first (at
-    // most 7); made with the handle, since a branch may run while a caller's stream is capturing
+    // The side streams of run_branches, as many as the step has branches beyond the first (at most
+    // 7); made with the handle, since a branch may run while a caller's stream is capturing. One
+    // costs 0.05 ms to make and as much to give back.
     void build_side_streams() {
-        size_t n = sb_.size() + fb_.size() + (ms_n_ || fs_n_) + 1;
-        if (cfg_.plain) n = 1;
-        n = std::min<size_t>(n - 1, 7);
-        AXG_CUDA(cudaEventCreateWithFlags(&fork_ev_, cudaEventDisableTiming));
-        for (size_t i = 0; i < n; i++) {
+        if (!fork_ev_) AXG_CUDA(cudaEventCreateWithFlags(&fork_ev_, cudaEventDisableTiming));
+        size_t n = cfg_.deterministic ? !sb_.empty() + !fb_.empty() : sb_.size() + fb_.size() + (ms_n_ || fs_n_);
+        n += has_records();
+        n = std::max<size_t>(n, (sp_.n > 0) + (fp_.n > 0));      // the point updates
+        n = cfg_.plain ? 1 : std::min<size_t>(n, 8);
+        while (side_.size() + 1 < n) {
             cudaStream_t q = nullptr;
             AXG_CUDA(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking));
             side_.push_back(q);
@@ -2132,6 +2121,8 @@ private:
             join_ev_.push_back(e);
         }
     }
+    bool has_records() const { return st_n_ || er_n_ || model_.scan.enabled; }
+
     // Independent launches of a step. Each branch is a chain of launches; the first stays on the
     // handle's stream, the others go round-robin to side streams that start after what is queued
     // so far and are joined before whatever follows (graph edges under capture). The buckets of a
@@ -2445,7 +2436,7 @@ private:
                 fluid_branches(br, -1);
                 if (ms_n_ || fs_n_) br.push_back([this] { launch_sources(); });
             }
-            if (st_n_ || er_n_ || model_.scan.enabled) br.push_back([this] { launch_records(); });
+            if (has_records()) br.push_back([this] { launch_records(); });
             run_branches(br);
         }
         launch_clayton();

@@ -607,12 +607,32 @@ __global__ void ocean3d_kernel(const Ocean3DArgs<T> a) {
 }
 
 // what the boundary conditions after assembly and the mass term do to one mode of one point
-// (AxialBoundary, FluidSurfaceBoundary, the Nyquist rule), formed once per mode on the host
+// (AxialBoundary, FluidSurfaceBoundary, the Nyquist rule), formed once per mode with the handle
 constexpr uint8_t MODE_SKIP = 1;    // Mass3D / ocean-load point: its own kernel does conditions and 1/M
 constexpr uint8_t MODE_AXIS0 = 2;   // solid axis, order 0: the horizontal components vanish
 constexpr uint8_t MODE_AXIS1 = 4;   // solid axis, order 1: horizontal components tied, vertical zero
 constexpr uint8_t MODE_ZERO = 8;    // higher orders on the axis, fluid surface
 constexpr uint8_t MODE_NYQUIST = 16;  // imaginary part dropped
+
+// the per-mode tables from the points, one thread per mode
+template <class T>
+__global__ void mode_table_kernel(int nmodes, bool solid, const int *mode_pt, const int *off, const int *nr,
+                                  const uint8_t *flags, const T *inv_mass1, uint8_t *mode_flags, T *mode_inv) {
+    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= nmodes) return;
+    const int p = mode_pt[m], al = m - off[p];
+    const uint8_t fl = flags[p];
+    uint8_t b = 0;
+    if (fl & (PT_MASS3D | PT_OCEAN)) b |= MODE_SKIP;
+    if (fl & PT_AXIAL) {
+        if (solid) b |= al == 0 ? MODE_AXIS0 : al == 1 ? MODE_AXIS1 : MODE_ZERO;
+        else if (al >= 1) b |= MODE_ZERO;
+    }
+    if (!solid && (fl & PT_SURFACE)) b |= MODE_ZERO;
+    if ((nr[p] & 1) == 0 && al == nr[p] / 2) b |= MODE_NYQUIST;
+    mode_flags[m] = b;
+    mode_inv[m] = inv_mass1[p];
+}
 
 template <class T, class D>
 struct PointArgs {
@@ -1163,6 +1183,12 @@ __global__ void narrow_kernel(const cx_t<D> *src, cx_t<T> *dst, size_t n) {
 template <class T>
 __global__ void set_step_kernel(int *step, int value) { *step = value; }
 
+// first mode and number of modes of every element point
+template <class T>
+__global__ void offset_table_kernel(int n, const int *pts, const int *off, const int *nu, int2 *tab) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) tab[i] = make_int2(off[pts[i]], nu[pts[i]]);
+}
 
 // ------------------------------------------------- boundary-stiffness exchange ---
 // MessageRank::gatherFromPoints / scatterToPoints (MessageRank.cpp:40-63) with

@@ -47,29 +47,33 @@ __host__ __device__ inline Tile1D<T, AT> tile_1d(int mt) {
     return L;
 }
 
-// SLS recursion of one (mode, point) with full attenuation, the steps of attenuate<>: two
-// groups of three stress components, the 3 + 3 NS state words of a group as complex loads in
-// flight together
+// SLS recursion of one (mode, point) with full attenuation, the steps of attenuate<>: groups of G
+// stress components, the G (1 + NS) state words of a group as complex loads in flight together. Two
+// components with five SLS hold as many words as three with three; three of them spilled 480 B in
+// FP32. Measured, 12 000 elements of nr up to 64 per step, G = 3 / 2 / 1: five SLS FP32 687 / 493 /
+// 715 us, FP64 state in FP32 elements 836 / 704 / 829 (FP64 985 / 817); three SLS FP32 371 / 404 /
+// 647, 553 / 559 / 756.
 template <int NS, class T, class AT>
 __device__ __forceinline__ void attenuate_full_1d(const SolidArgs<T, AT> &a, cx_t<AT> *st, size_t nslot,
                                                   const cx_t<T> (&e)[6], cx_t<T> (&s)[6], T dl, T dm) {
     using CA = cx_t<AT>;
+    constexpr int G = NS > 3 ? 2 : 3;
     const AT lam = (AT)dl, mu = (AT)dm, mu2 = mu + mu;
     const CA tr = mk<AT>(((AT)e[0].x + (AT)e[1].x + (AT)e[2].x) * lam, ((AT)e[0].y + (AT)e[1].y + (AT)e[2].y) * lam);
 #pragma unroll
-    for (int g = 0; g < 2; g++) {
-        CA ds[3], mem[NS][3];
+    for (int g = 0; g < 6 / G; g++) {
+        CA ds[G], mem[NS][G];
 #pragma unroll
-        for (int c = 0; c < 3; c++) ds[c] = st[(3 * g + c) * nslot];
+        for (int c = 0; c < G; c++) ds[c] = st[(G * g + c) * nslot];
 #pragma unroll
         for (int l = 0; l < NS; l++)
 #pragma unroll
-            for (int c = 0; c < 3; c++) mem[l][c] = st[(6 + l * 6 + 3 * g + c) * nslot];
+            for (int c = 0; c < G; c++) mem[l][c] = st[(6 + l * 6 + G * g + c) * nslot];
 #pragma unroll
-        for (int c = 0; c < 3; c++) {
-            const int d = 3 * g + c;
+        for (int c = 0; c < G; c++) {
+            const int d = G * g + c;
             const CA ed = mk<AT>((AT)e[d].x, (AT)e[d].y);
-            const CA dn = g == 0 ? mk<AT>(tr.x + ed.x * mu2, tr.y + ed.y * mu2) : mk<AT>(ed.x * mu, ed.y * mu);
+            const CA dn = d < 3 ? mk<AT>(tr.x + ed.x * mu2, tr.y + ed.y * mu2) : mk<AT>(ed.x * mu, ed.y * mu);
             CA sv = mk<AT>((AT)s[d].x, (AT)s[d].y);
             st[d * nslot] = dn;
 #pragma unroll

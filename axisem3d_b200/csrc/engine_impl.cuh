@@ -561,6 +561,7 @@ public:
         ensure_capacity(step_ + nsteps);
         const size_t nf = (size_t)sp_.total * 3;
         const int nck = (nsteps + interval - 1) / interval;
+        ck_n_ = 0;   // no run to go back over until all of its checkpoints have their place
         ck_displ_.fit(nf * nck); ck_veloc_.fit(nf * nck); ck_accel_.fit(nf * nck);
         if (state_wave_ > 0) ck_state_.fit((size_t)state_wave_ * nck);
         ck_n_ = nsteps; ck_interval_ = interval; ck_step0_ = step_;

@@ -165,3 +165,23 @@ def test_hooks_runs_and_streams_in_turn(built):
         d, g = s.get_field("displ"), s.seismograms()
     assert np.linalg.norm(d - ref) <= 1e-12 * np.linalg.norm(ref)
     assert np.linalg.norm(g[:seis.shape[0]] - seis) <= 1e-12 * np.linalg.norm(seis)
+
+
+def test_adjoint_after_checkpoints_that_did_not_fit(built):
+    """Checkpoints beyond the GPU's memory are refused, and the run before them, whose checkpoints gave
+    way, cannot be gone back over."""
+    from axisem3d_b200 import _lib as L
+    m = meshgen.cartesian_model(nx=8, nz=8, nr=9, nstations=2, record_interval=10 ** 6)
+    with Solver(m, "fp64") as s:
+        s.forward_checkpointed(4, 2)
+        seis = s.seismograms()
+        n = int(4e11 / (16 * s.field_size()))          # 400 GB of displacement alone
+        with pytest.raises(EngineError) as ei:
+            s.forward_checkpointed(n, 1)
+        assert ei.value.code == L.AXG_E_NOMEM
+        with pytest.raises(EngineError) as ei:
+            s.adjoint(seis)
+        assert ei.value.code == L.AXG_E_STATE
+        s.forward_checkpointed(4, 2)
+        g = s.adjoint(s.seismograms())
+    assert np.all(np.isfinite(g["moduli"]))

@@ -1,5 +1,5 @@
 """What handles choose for themselves, and what those of one process share or keep between calls: the
-autotuner's team sizes, the captured steps, the step counter and the tables of a hook loop, the
+autotuner's team sizes, the captured steps (their own and a caller's), the step counter and the tables of a hook loop, the
 runtime's record of an error."""
 import time
 
@@ -30,20 +30,33 @@ def test_a_failed_call_does_not_fail_the_next_one(built):
     assert np.linalg.norm(d - e) <= 1e-13 * np.linalg.norm(e)
 
 
+def _captured_stiffness(s, *buffers):
+    """One no-allocation stiffness evaluation of the device buffers x, f (and of the fluid's) as a
+    captured graph of the caller's stream."""
+    import torch
+    stream = torch.cuda.Stream()
+    s.set_stream(stream.cuda_stream)
+    torch.cuda.synchronize()
+    ptr = [b.data_ptr() for b in buffers]
+    s.compute_stiffness_noalloc(*ptr)      # looks the library's array up
+    stream.synchronize()
+    g = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(g, stream=stream):
+        s.compute_stiffness_noalloc(*ptr)
+    return g, stream
+
+
+def _on_device(u, dtype):
+    import torch
+    return torch.view_as_real(torch.from_numpy(u).to("cuda", dtype)).contiguous()
+
+
 def _block_threads(s, u):
     """Threads per block of the kernels of one stiffness evaluation, from a captured graph of it."""
     import torch
     from cuda.bindings import driver
-    x = torch.view_as_real(torch.from_numpy(u).to("cuda")).contiguous()
-    f = torch.zeros_like(x)
-    stream = torch.cuda.Stream()
-    s.set_stream(stream.cuda_stream)
-    torch.cuda.synchronize()
-    s.compute_stiffness_noalloc(x.data_ptr(), f.data_ptr())      # looks the library's array up
-    stream.synchronize()
-    g = torch.cuda.CUDAGraph(keep_graph=True)
-    with torch.cuda.graph(g, stream=stream):
-        s.compute_stiffness_noalloc(x.data_ptr(), f.data_ptr())
+    x = _on_device(u, torch.complex128)
+    g, stream = _captured_stiffness(s, x, torch.zeros_like(x))
     graph = driver.CUgraph(g.raw_cuda_graph())
     count = driver.cuGraphGetNodes(graph)[2]
     threads = []
@@ -185,3 +198,35 @@ def test_adjoint_after_checkpoints_that_did_not_fit(built):
         s.forward_checkpointed(4, 2)
         g = s.adjoint(s.seismograms())
     assert np.all(np.isfinite(g["moduli"]))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_captured_stiffness_of_several_buckets(built, precision):
+    """A caller's capture takes the branches of every bucket, solid and fluid, into its graph; a replay
+    on other inputs in the same buffers gives the handle's own stiffness."""
+    import torch
+    m = meshgen.spherical_model(n_theta=24, n_solid_layers=6, n_fluid_layers=2, nr_max=40)
+    dtype = torch.complex128 if precision == "fp64" else torch.complex64
+    us, uf = meshgen.random_displacement(m, seed=5), meshgen.random_displacement(m, seed=6, solid=False)
+    with Solver(m, precision) as s:
+        s.set_field(us, "displ")
+        s.set_field(uf, "displ", solid=False)
+        s.compute_stiffness()
+        ref = s.get_field("stiff"), s.get_field("stiff", solid=False)
+    with Solver(m, precision) as s:
+        x, y = _on_device(0 * us, dtype), _on_device(0 * uf, dtype)
+        f, h = torch.zeros_like(x), torch.zeros_like(y)
+        g, stream = _captured_stiffness(s, x, f, y, h)
+        x.copy_(_on_device(us, dtype))
+        y.copy_(_on_device(uf, dtype))
+        for _ in range(2):
+            f.zero_()
+            h.zero_()
+            torch.cuda.synchronize()
+            with torch.cuda.stream(stream):
+                g.replay()
+            torch.cuda.synchronize()
+        got = [torch.view_as_complex(t).cpu().numpy() for t in (f, h)]
+        s.set_stream(None)
+    for a, b in zip(got, ref):
+        assert np.linalg.norm(a.ravel() - b) <= (1e-12 if precision == "fp64" else 1e-6) * np.linalg.norm(b)

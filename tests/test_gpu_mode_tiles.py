@@ -57,6 +57,10 @@ def test_cg4_tiles_match_oracle(built, precision, nr):
     f, d = _oracle_steps(m, u, 5)
     with Solver(m, precision) as s:
         s.set_field(u, "displ")
+        s.compute_stiffness()
+        assert np.linalg.norm(s.get_field("stiff") - f) <= TOL[precision] * np.linalg.norm(f)
+    with Solver(m, precision) as s:
+        s.set_field(u, "displ")
         s.run(5)
         assert np.linalg.norm(s.get_field("displ") - d) <= TOL[precision] * np.linalg.norm(d)
 
@@ -79,6 +83,32 @@ def test_waves_split_over_blocks(built, nwave):
         got = s.get_field("displ").reshape(nwave, -1)
     for w in range(nwave):
         assert np.linalg.norm(got[w] - one[w]) <= 1e-13 * np.linalg.norm(one[w])
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("attenuation, nrs", [("full", [9, 17, 30, 34]), ("full", [70, 96]), ("cg4", [64])])
+def test_attenuating_slices_split_over_blocks(built, attenuation, nrs, precision):
+    """The same for 3-D elements with attenuation: every wavefield of a batch has its own memory
+    variables."""
+    nwave = 5
+    m = meshgen.microbench_model(n_elem=6, nr_choices=nrs, attenuation=attenuation, seed=7)
+    us = [meshgen.random_displacement(m, seed=10 + w) for w in range(nwave)]
+    one = []
+    for u in us:
+        with Solver(m, precision) as s:
+            s.set_field(u, "displ")
+            s.run(4)
+            s.compute_stiffness()
+            one.append((s.get_field("displ"), s.get_field("stiff")))
+    m.nwave = nwave
+    with Solver(m, precision) as s:
+        s.set_field(np.concatenate(us), "displ")
+        s.run(4)
+        s.compute_stiffness()
+        got = [s.get_field(k).reshape(nwave, -1) for k in ("displ", "stiff")]
+    for w in range(nwave):
+        for g, ref in zip(got, one[w]):
+            assert np.linalg.norm(g[w] - ref) <= TOL[precision] * np.linalg.norm(ref)
 
 
 def test_handles_of_two_precisions_share_kernels(built):
@@ -129,14 +159,18 @@ def test_cg4_slices_match_oracle(built, nr):
     for teams in (None, {3: 128, 4: 128}):
         with Solver(m, "mixed", team_sizes=teams) as s:
             s.set_field(u, "displ")
+            s.compute_stiffness()
+            assert np.linalg.norm(s.get_field("stiff") - f) <= TOL["mixed"] * np.linalg.norm(f)
+        with Solver(m, "mixed", team_sizes=teams) as s:
+            s.set_field(u, "displ")
             s.run(4)
             assert np.linalg.norm(s.get_field("displ") - d) <= TOL["mixed"] * np.linalg.norm(d)
 
 
 @pytest.mark.parametrize("pieces", [[64], [1, 7, 8, 48], [15, 16, 17, 16], [33, 31]])
 def test_step_graphs_of_one_and_several_steps(built, pieces):
-    """Runs of any length replay graphs of eight steps and of one: the same steps, records and
-    source times as launch by launch."""
+    """Runs of any length replay captured steps: the same steps, records and source times as launch by
+    launch."""
     m = meshgen.cartesian_model(nx=7, nz=5, nr=5, nstations=4, record_interval=3)
     with Solver(m, "fp64") as s:
         s.run(64, graph=False)
@@ -177,6 +211,10 @@ def test_small_buckets_largest_elements_first(built, precision):
     m = meshgen.microbench_model(n_elem=40, nr_min=26, nr_max=64, seed=17)
     u = meshgen.random_displacement(m, seed=8)
     f, d = _oracle_steps(m, u, 4)
+    with Solver(m, precision) as s:
+        s.set_field(u, "displ")
+        s.compute_stiffness()
+        assert np.linalg.norm(s.get_field("stiff") - f) <= TOL[precision] * np.linalg.norm(f)
     with Solver(m, precision) as s:
         s.set_field(u, "displ")
         s.run(4)

@@ -321,16 +321,19 @@ public:
                 launches_ += kernels_per_step_ * steps;
                 left -= steps;
             };
-            // Several steps in one graph where a handle runs enough of them: a graph's start and end
-            // cost a small mesh's step about as much as one of its kernels. Building it is host time,
-            // so the steps ahead of it are queued first and the GPU runs them meanwhile.
-            if (nsteps >= kGraphSteps) asked_ += nsteps;
-            if (asked_ >= kManySteps && nsteps >= kGraphSteps) {
+            // Several steps in one graph where that repays the building, which is host time: the steps
+            // ahead of it are queued first and the GPU runs them meanwhile.
+            if (nsteps >= kGraphSteps) {
+                asked_ += nsteps;
                 if (!many_.exec) {
-                    for (int k = 0; k < kLeadSteps && left > 0; k++) replay(one_, 1);
-                    refresh(many_, kGraphSteps);
+                    refresh(one_, 1);
+                    const int lead = lead_steps();
+                    if (asked_ >= kManySteps || nsteps >= lead + kGraphSteps) {
+                        for (int k = 0; k < std::min(lead, kLeadSteps) && left > 0; k++) replay(one_, 1);
+                        refresh(many_, kGraphSteps);
+                    }
                 }
-                while (left >= kGraphSteps) replay(many_, kGraphSteps);
+                while (many_.exec && left >= kGraphSteps) replay(many_, kGraphSteps);
             }
             while (left > 0) replay(one_, 1);
         } else {
@@ -2457,14 +2460,23 @@ private:
             throw Error(AXG_E_CUDA, std::string("Engine::launch || ") + cudaGetErrorString(e));
     }
 
-    // Captured steps. The graph of eight of them costs a small mesh 0.7 (40 x 40 box) to 1.4 ms (1-D
-    // globe, 9 launches per step) to instantiate and about as much to destroy, and saves 3.5 and 10 us
-    // a step: it is made once a handle has been asked for kManySteps steps in runs that can use it,
-    // behind kLeadSteps queued ones. Made in every run of 16 steps or more, and again at each growth
-    // of the tables, it cost the first three runs of 20 steps 1.1, 1.9 and 1.9 ms on the box and 2.5,
-    // 4.1 and 4.4 on the globe; this way 0.6, 0.4, 0.4 and 1.6, 1.1, 1.5, and 100 steps of a handle
-    // in use are what they were (1.35 and 4.60 ms).
+    // Captured steps. The graph of eight of them takes the host 0.7 (40 x 40 box) to 1.4 ms (1-D globe, 9
+    // launches per step) to instantiate and about as much to destroy, and saves 3.5 and 10 us a step
+    // (5 of 326 on the FP32 block mesh). It is made in the first run whose steps ahead of it keep the
+    // GPU busy that long, else once a handle has been asked for kManySteps steps in runs that can use
+    // it. Made in every run of 16 steps or more, and again at each growth of the tables, it cost the
+    // first three runs of 20 steps 1.1, 1.9 and 1.9 ms on the box and 2.5, 4.1 and 4.4 on the globe;
+    // this way 0.6, 0.4, 0.4 and 1.6, 1.1, 1.5, and 100 steps of a handle in use are what they were
+    // (1.35 and 4.60 ms).
     static constexpr int kGraphSteps = 8, kManySteps = 256, kLeadSteps = 64;
+    // steps that cover the building of many_ by themselves: 20 us a launch (measured 9 - 20), against
+    // the bytes of a step at 6.5 TB/s, which none is faster than
+    int lead_steps() const {
+        double b = 0, f = 0;
+        stiffness_cost(&b, &f);
+        const double step_us = (b + point_cost()) / 6.5e6, build_us = 20. * kGraphSteps * (double)kernels_per_step_;
+        return (int)std::ceil(build_us / std::max(step_us, 0.1));
+    }
     struct StepGraph {
         cudaGraphExec_t exec = nullptr;
         bool stale = true;    // a table of the step has moved since the capture

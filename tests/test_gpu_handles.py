@@ -98,6 +98,21 @@ def test_graph_of_several_steps_behind_single_ones(built, pieces):
     assert g.shape == seis.shape and np.linalg.norm(g - seis) <= 1e-11 * np.linalg.norm(seis)
 
 
+def test_graph_of_several_steps_in_a_first_run(built):
+    """On a mesh whose steps cover the building, a first run of 20 steps has the graph of eight too."""
+    m = meshgen.microbench_model(n_elem=1500, nr_choices=[40], rheology="iso", attenuation="full", seed=6)
+    u = meshgen.random_displacement(m, seed=4)
+    out = []
+    for graph in (False, True):
+        with Solver(m, "fp64") as s:
+            s.set_field(u, "displ")
+            for n in (20, 13):
+                s.run(n, graph=graph)
+            assert s.step == 33
+            out.append(s.get_field("displ"))
+    assert np.linalg.norm(out[1] - out[0]) <= 1e-11 * np.linalg.norm(out[0])
+
+
 def test_short_runs_do_not_pay_for_graphs(built):
     """Runs of 20 steps of a new handle, the tables growing under them, take no longer than twice
     their launches one by one (three to four times with graphs of eight steps made for each)."""

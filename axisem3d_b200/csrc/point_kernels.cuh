@@ -655,11 +655,11 @@ struct PointArgs {
 };
 
 // One thread per complex value of the point fields ([nmodes][ndim], a wavefield per (y, z)
-// block index), so that every field is read and written in consecutive 8- / 16-byte words. The only condition
-// that mixes the components of a mode (the axial order-1 rule) reads the other component before
-// the block's barrier and every thread writes after it; blocks of POINT_BLOCK threads hold whole
-// modes. Bound by HBM: 128 bytes per complex value in the mixed mode. The conditions and 1/M
-// come from per-mode tables, so that no load of a thread waits on another: all of them are in
+// block index), so that every field is read and written in consecutive 8- / 16-byte words. The only
+// condition that mixes the components of a mode (the axial order-1 rule) reads the other component
+// before the block's barrier and every thread writes after it; blocks of POINT_BLOCK threads hold
+// whole modes. Bound by HBM: 136 bytes per complex value in the mixed mode with compensation, 104
+// without. The conditions and 1/M come from per-mode tables, so that no load of a thread waits on another: all of them are in
 // flight at once (through the point of the mode, its offset, order, flags and mass followed one
 // another in three dependent rounds before the fields were asked for).
 constexpr int POINT_BLOCK = 288;   // 96 modes of 3 components, 9 warps

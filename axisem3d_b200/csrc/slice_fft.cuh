@@ -8,10 +8,11 @@
 //
 // The transform is a mixed-radix Stockham FFT, one pass over shared memory per factor of nr, and a
 // pass costs a barrier of the team, a read and a write of every sample and the index arithmetic,
-// whatever its radix. So the factors are as few and as even as they go: radices up to 16, each a
-// DFT in registers (of its prime factors, constants folded in), which makes nr = 2 .. 128 two passes
-// where prime radices took up to six. The transforms of both directions run with the positive
-// sign: the spectrum of (x_2p+1, x_2p), real and imaginary part exchanged, is the exchanged
+// whatever its radix. So the factors are as few and as even as they go: radices up to 16 (FP64: 10, 11
+// and 13), each a DFT in registers (of its prime factors, constants folded in). An nr of 26 .. 128
+// without a prime factor above 13 takes two passes in FP32 (125 three) where prime radices took up to
+// six; in FP64 75, 84, 96, 98, 105, 108, 112, 120, 126 and 128 take three as well. The transforms of
+// both directions run with the positive sign: the spectrum of (x_2p+1, x_2p), real and imaginary part exchanged, is the exchanged
 // spectrum of the negative sign.
 #pragma once
 

@@ -1,7 +1,7 @@
 """A whole simulation from the reference's inputs: preloop, time loop on the GPU, station
 files. This is the path of the reference's `main` (SOLVER/src/main.cpp): the inputs
 (inparam.*.yaml and the Exodus mesh they name) go through `preloop.build`, the Newmark loop
-runs in the engine (one CUDA graph per step), and each station group is written in its
+runs in the engine (captured CUDA graphs of the step), and each station group is written in its
 format (`output.write_group`).
 
     from axisem3d_b200 import simulation

@@ -12,7 +12,7 @@ inverse transform, quadrature, scatter-add), then boundary conditions, 1/M and
 the Newmark update. Updates per step = sum_e 25 nu_e (nu = nr/2 + 1).
 
   value  device-timed with CUDA events on the engine's stream, state resident in
-         HBM, one CUDA graph per step; inputs larger than L2 (the step streams
+         HBM, replayed from CUDA graphs; inputs larger than L2 (the step streams
          ~20 GB)
   e2e    the same steps through the C ABI with the displacement field copied
          host -> device from pinned memory before every step and the updated
@@ -466,7 +466,7 @@ def ensemble_timing(args, local, stream, world):
     """Batched ensemble: `--ensemble` moment-tensor sources (Ricker, periods 10-40 s) with
     full 21-Cij on a spherical-shell mesh (8000 solid + 400 fluid quads, r 3480-6371 km,
     fluid 3480-3600 km, nr 3..100 from a 2 % dlnVs random field, elastic, RTZ frame),
-    all advanced as one wavefield batch per launch, one CUDA graph per step, autotuned
+    all advanced as one wavefield batch per launch, replayed from CUDA graphs, autotuned
     team sizes, in the bench precision; against the plain FP64 method (one bucket per
     material kind, eager launches) advancing one of the sources on the same mesh."""
     from axisem3d_b200 import meshgen
@@ -575,7 +575,7 @@ def main():
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
             "dtype": {"mixed": "f32 (f64 Newmark d/v and SLS state)", "fp32": "f32", "fp64": "f64"}[args.precision],
             "data": "synthetic", "config": workload_config(args, m),
-            "precision": args.precision, "graph": "one CUDA graph per step",
+            "precision": args.precision, "graph": "CUDA graphs of one or eight steps",
             "gpu_launches": int(r["launches"]),
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic,

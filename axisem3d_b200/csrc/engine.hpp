@@ -187,7 +187,7 @@ struct HostModel {
 class EngineBase {
 public:
     virtual ~EngineBase() = default;
-    virtual void finalize(const HostModel &m) = 0;
+    virtual void finalize(HostModel &m) = 0;
     virtual void apply_sources(int tstep) = 0;
     virtual void compute_stiffness() = 0;
     virtual void compute_stiffness_part(int part) = 0;   // the buckets of one element part

@@ -212,8 +212,20 @@ public:
     }
 
     // ------------------------------------------------------------ finalize ---
-    void finalize(const HostModel &m) override {
-        model_ = m;
+    // takes the model over; it is the caller's again if the handle cannot be made
+    void finalize(HostModel &m) override {
+        std::swap(model_, m);
+        try {
+            build(model_);
+        } catch (...) {
+            std::swap(model_, m);
+            throw;
+        }
+        finalized_ = true;
+    }
+
+private:
+    void build(const HostModel &m) {
         const SpectralTables &st = spectral_tables();
         std::vector<T> g(50);
         for (int i = 0; i < 25; i++) { g[i] = (T)st.G_GLL[i]; g[25 + i] = (T)st.G_GLJ[i]; }
@@ -271,8 +283,9 @@ public:
         AXG_CUDA(cudaEventCreate(&ev1_));
         build_side_streams();
         AXG_CUDA(cudaStreamSynchronize(stream_));
-        finalized_ = true;
     }
+
+public:
 
     // ------------------------------------------------------------ hooks ---
     void apply_sources(int tstep) override {
@@ -1154,7 +1167,7 @@ private:
         P.n = h.count;
         P.ndim = solid ? 3 : 1;
         P.h_off.resize(P.n); P.h_nu.resize(P.n); P.h_nr.resize(P.n);
-        std::vector<int> mode_pt, pt3d;
+        std::vector<int> pt3d;
         std::vector<uint8_t> flags(P.n, 0);
         std::vector<T> inv1(P.n, (T)0), inv3;
         std::vector<int64_t> im_off(P.n, 0);
@@ -1163,7 +1176,6 @@ private:
             int nr = h.nr[p];
             if (nr < 1) throw Error(AXG_E_ARG, "Point::Point || nr must be >= 1.");
             P.h_nr[p] = nr; P.h_nu[p] = nr / 2 + 1; P.h_off[p] = o;
-            for (int a = 0; a < P.h_nu[p]; a++) mode_pt.push_back(p);
             o += P.h_nu[p];
             P.nr_max = std::max(P.nr_max, nr);
             int mnr = h.mass_nr.size() ? h.mass_nr[p] : 1;
@@ -1181,6 +1193,8 @@ private:
             if (h.surface.size() && h.surface[p]) flags[p] |= PT_SURFACE;
         }
         P.total = o;
+        std::vector<int> mode_pt(P.total);
+        for (int p = 0; p < P.n; p++) std::fill_n(mode_pt.begin() + P.h_off[p], P.h_nu[p], p);
         P.n3d = (int)pt3d.size();
         P.off.upload(P.h_off); P.nu.upload(P.h_nu); P.nr.upload(P.h_nr);
         P.mode_pt.upload(mode_pt); P.pt3d.upload(pt3d);

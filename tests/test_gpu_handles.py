@@ -245,3 +245,21 @@ def test_captured_stiffness_of_several_buckets(built, precision):
         s.set_stream(None)
     for a, b in zip(got, ref):
         assert np.linalg.norm(a.ravel() - b) <= (1e-12 if precision == "fp64" else 1e-6) * np.linalg.norm(b)
+
+
+def test_a_handle_that_cannot_be_made_keeps_its_model(built):
+    """axg_finalize takes the model over; refused (modes that no block holds), it is refused again and
+    not made of an empty one."""
+    from axisem3d_b200 import _lib as L
+
+    class Unchecked(Solver):
+        def _check(self, rc):
+            self.rc = rc
+
+    m = meshgen.microbench_model(n_elem=2, nr_choices=[260], rheology="iso", attenuation=None)
+    s = Unchecked(m, "fp64")
+    assert s.rc == L.AXG_E_UNSUPPORTED
+    assert s.lib.axg_finalize(s.h) == L.AXG_E_UNSUPPORTED
+    assert b"too large" in s.lib.axg_last_error(s.h)
+    assert s.lib.axg_run(s.h, 1, 1) == L.AXG_E_STATE
+    s.close()

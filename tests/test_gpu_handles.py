@@ -118,7 +118,7 @@ def test_short_runs_do_not_pay_for_graphs(built):
     their launches one by one (three to four times with graphs of eight steps made for each)."""
     m = meshgen.cartesian_model(nx=40, nz=40, nr=5, nstations=20)
     best = {}
-    for graph in (False, True) * 4:
+    for graph in (False, True) * 8:
         with Solver(m, "fp32") as s:
             s.run(20, graph=graph)
             s.synchronize()

@@ -291,6 +291,7 @@ public:
     void apply_sources(int tstep) override {
         need();
         if (tstep < 0) throw Error(AXG_E_ARG, "Domain::applySources || negative time step.");
+        need_no_capture();
         ensure_capacity(tstep + 1);   // the STF table must cover this step
         set_step(tstep);
         launch_sources();
@@ -306,6 +307,7 @@ public:
     void record(int tstep) override {
         need();
         if (tstep < 0) throw Error(AXG_E_ARG, "Domain::recordOutput || negative time step.");
+        need_no_capture();
         ensure_capacity(tstep + 1);
         set_step(tstep);
         launch_records();
@@ -314,6 +316,7 @@ public:
     void run(int nsteps, bool graph) override {
         need();
         if (nsteps <= 0) return;
+        need_no_capture();
         ensure_capacity(step_ + nsteps);
         set_step(step_);
         dev_step_ = -1;   // the steps advance it; known again when all of them are queued
@@ -574,6 +577,7 @@ public:
             throw Error(AXG_E_UNSUPPORTED, "axg_forward_checkpointed || needs an FP64 handle.");
         check_adjoint_model();
         if (nsteps <= 0 || interval <= 0) throw Error(AXG_E_ARG, "axg_forward_checkpointed || bad sizes.");
+        need_no_capture();
         ensure_capacity(step_ + nsteps);
         const size_t nf = (size_t)sp_.total * 3;
         const int nck = (nsteps + interval - 1) / interval;
@@ -1088,13 +1092,18 @@ private:
     void need() const {
         if (!finalized_) throw Error(AXG_E_STATE, "Engine::step || axg_finalize not called.");
     }
-    // the device step counter, set by a one-thread kernel when it does not hold the step already
-    // (a copy from the host and its synchronisation took two round trips of every hook-driven step)
-    void set_step(int tstep) {
+    // What sets the step or grows a table is refused while the handle's stream is capturing, before it
+    // does anything that would break the caller's capture.
+    void need_no_capture() const {
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         AXG_CUDA(cudaStreamIsCapturing(stream_, &cap));
         if (cap != cudaStreamCaptureStatusNone)
             throw Error(AXG_E_CUDA, "Engine::set_step || the time step cannot be set while the stream is capturing.");
+    }
+    // the device step counter, set by a one-thread kernel when it does not hold the step already
+    // (a copy from the host and its synchronisation took two round trips of every hook-driven step)
+    void set_step(int tstep) {
+        need_no_capture();
         if (dev_step_ == tstep) return;
         set_step_kernel<T><<<1, 1, 0, stream_>>>(step_dev_.p, tstep);
         AXG_CUDA(cudaGetLastError());

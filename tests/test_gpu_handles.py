@@ -263,3 +263,38 @@ def test_a_handle_that_cannot_be_made_keeps_its_model(built):
     assert b"too large" in s.lib.axg_last_error(s.h)
     assert s.lib.axg_run(s.h, 1, 1) == L.AXG_E_STATE
     s.close()
+
+
+def test_refused_hooks_leave_a_capture_alone(built):
+    """The hooks that set the step, and runs, are refused while the caller's stream is capturing, also
+    where they would have to grow a table first; the capture goes on and its graph is whole."""
+    import torch
+    m = meshgen.cartesian_model(nx=6, nz=5, nr=5, nstations=2)
+    u = meshgen.random_displacement(m, seed=9)
+    with Solver(m, "fp64") as s:
+        s.set_field(u, "displ")
+        s.compute_stiffness()
+        ref = s.get_field("stiff")
+    with Solver(m, "fp64") as s:
+        x = _on_device(u, torch.complex128)
+        f = torch.zeros_like(x)
+        stream = torch.cuda.Stream()
+        s.set_stream(stream.cuda_stream)
+        torch.cuda.synchronize()
+        s.compute_stiffness_noalloc(x.data_ptr(), f.data_ptr())
+        stream.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=stream, capture_error_mode="thread_local"):
+            s.compute_stiffness_noalloc(x.data_ptr(), f.data_ptr())
+            for call in (lambda: s.apply_sources(100), lambda: s.record_stations(100), lambda: s.run(20)):
+                with pytest.raises(EngineError, match="capturing"):
+                    call()
+        f.zero_()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(stream):
+            g.replay()
+        torch.cuda.synchronize()
+        got = torch.view_as_complex(f).cpu().numpy().ravel()
+        s.set_stream(None)
+        s.run(4)
+    assert np.linalg.norm(got - ref) <= 1e-12 * np.linalg.norm(ref)
